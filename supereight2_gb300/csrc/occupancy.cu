@@ -299,6 +299,39 @@ __device__ __forceinline__ bool occ_interp(const OccDevice& m, OccCursor& c, con
     return ok;
 }
 
+// Whether occ_interp has a value at vf, by one lane alone.
+__device__ __forceinline__ bool occ_interp_exists(const OccDevice& m, OccCursor& c, const int* aabb, F3 vf)
+{
+    const int q = occ_seek(m, c, (int) vf.x, (int) vf.y, (int) vf.z);
+    if (q == -1)
+        return false;
+    bool valid = false;
+#pragma unroll 1
+    for (int scale = slot_is_block(q) ? c.cur : 0; scale <= kOccMaxScale; ++scale) {
+        const int stride = 1 << scale;
+        const float inv = occ_inv_size(scale);
+        const int b0 = stride * (int) (inv * vf.x - 0.5f), b1 = stride * (int) (inv * vf.y - 0.5f),
+                  b2 = stride * (int) (inv * vf.z - 0.5f);
+        if (aabb[6] || b0 < aabb[0] || b1 < aabb[1] || b2 < aabb[2] || b0 > aabb[3] || b1 > aabb[4] || b2 > aabb[5])
+            break;
+        if (b0 + stride >= m.size || b1 + stride >= m.size || b2 + stride >= m.size || b0 < 0 || b1 < 0 || b2 < 0)
+            continue;
+        bool have = true;
+        valid = true;
+#pragma unroll 1
+        for (int k = 0; k < 8 && have; ++k) {
+            OccD e = occ_default();
+            have = occ_data_at(m, c, b0 + ((k & 1) ? stride : 0), b1 + ((k & 2) ? stride : 0), b2 + ((k & 4) ? stride : 0), scale,
+                               e);
+            valid = valid && occ_valid(e);
+        }
+        if (have)
+            break;
+        valid = false;
+    }
+    return valid;
+}
+
 // The 32 gradient samples in the reference's order: per axis a selector of {base - stride, base,
 // base + stride, base + 2 stride}, packed x | y << 2 | z << 4.
 static __constant__ unsigned char kOccGradSel[32] = {
@@ -581,6 +614,11 @@ __device__ __forceinline__ bool occ_raycast(const OccDevice& m, OccCursor& c, co
     hit = f3(0.0f, 0.0f, 0.0f);
     bool want = false; // the sample at t waits for its interpolation
     float value = 0.0f;
+    // interpolations that the search made in a row without a value: along the edge of what has been seen a
+    // ray meets hundreds of such points (up to 269 in a view of the room), so after kOccTries each lane
+    // looks for itself whether its sample has one
+    constexpr int kOccTries = 2;
+    int failed = 0;
     for (;;) {
         const bool take = mode != kDone && !want, find = mode == kFind;
         float tk = t; // sample `lane`, its steps accumulated one by one
@@ -603,6 +641,8 @@ __device__ __forceinline__ bool occ_raycast(const OccDevice& m, OccCursor& c, co
                 fk = occ_field(data);
                 if (find && !has && lane == 7 && !slot_is_block(c.slot))
                     pass = occ_box_steps(c, vk, dv, step);
+                if (find && has && failed >= kOccTries)
+                    has = occ_interp_exists(m, c, aabb, vk);
             }
         }
         const unsigned events = occ_votes(take && there && (find ? has : !has || fk > -0.2f));
@@ -675,6 +715,7 @@ __device__ __forceinline__ bool occ_raycast(const OccDevice& m, OccCursor& c, co
             continue;
         want = false;
         if (mode == kFind) {
+            failed = ok ? 0 : failed + 1;
             if (ok) {
                 t_pt = t;
                 value_t = value;
