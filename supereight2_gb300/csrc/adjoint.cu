@@ -26,16 +26,62 @@
 
 namespace se_gpu {
 
-// The 8 corners of a trilinear sample, with what the adjoint needs.
+// The 8 corners of a trilinear sample, with what the adjoint needs. The corners stay from sample to sample:
+// the root search takes most of its samples in one cell.
 struct Tri {
-    int blk[8];
-    short vi[8];
+    int b0, b1, b2; // the cell of the corners, b0 < 0: none
+    int blk[8];     // the corners' blocks
     float f[8];
     F3 t; // fractional position in the cell
 };
 
+__device__ __forceinline__ int tri_voxel(const Tri& q, int n)
+{
+    return ((q.b0 + (n & 1)) & 7) + 8 * ((q.b1 + ((n >> 1) & 1)) & 7) + 64 * ((q.b2 + (n >> 2)) & 7);
+}
+
+// The corners of cell (b0, b1, b2) (inside the map): their block lookups in flight together, then their
+// voxels. (One corner after another, and all of them for each sample of the root search, a 640x480 render at
+// 1 cm took 283 us and its adjoint 376; so 128 and 150.)
 template <int S>
-__device__ bool tri_sample(const MapDevice& m, BlockCache& c, F3 p_W, Tri& q, float& value)
+__device__ __forceinline__ bool tri_load(const MapDevice& m, Tri& q, int b0, int b1, int b2)
+{
+    q.b0 = b0;
+    q.b1 = b1;
+    q.b2 = b2;
+    bool ok = true;
+    if ((b0 & 7) != 7 && (b1 & 7) != 7 && (b2 & 7) != 7) {
+        const int blk = __ldg(&m.block_index[((size_t) (b2 >> 3) << (2 * m.log2_bps)) | ((size_t) (b1 >> 3) << m.log2_bps)
+                                             | (size_t) (b0 >> 3)]);
+        ok = blk >= 0;
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+            q.blk[n] = blk;
+    }
+    else {
+#pragma unroll
+        for (int n = 0; n < 8; ++n) {
+            const int vx = b0 + (n & 1), vy = b1 + ((n >> 1) & 1), vz = b2 + (n >> 2);
+            q.blk[n] = __ldg(&m.block_index[((size_t) (vz >> 3) << (2 * m.log2_bps)) | ((size_t) (vy >> 3) << m.log2_bps)
+                                            | (size_t) (vx >> 3)]);
+            ok = ok && q.blk[n] >= 0;
+        }
+    }
+    if (ok) {
+#pragma unroll
+        for (int n = 0; n < 8; ++n) {
+            float w;
+            load_voxel<S>(m, q.blk[n], tri_voxel(q, n), q.f[n], w);
+            ok = ok && (w != 0.0f);
+        }
+    }
+    if (!ok)
+        q.b0 = -1;
+    return ok;
+}
+
+template <int S>
+__device__ __forceinline__ bool tri_sample(const MapDevice& m, F3 p_W, Tri& q, float& value)
 {
     F3 vf;
     if (!point_to_voxel_f(m, p_W, vf))
@@ -44,20 +90,8 @@ __device__ bool tri_sample(const MapDevice& m, BlockCache& c, F3 p_W, Tri& q, fl
     const int b0 = (int) bf.x, b1 = (int) bf.y, b2 = (int) bf.z;
     if (b0 < 0 || b1 < 0 || b2 < 0 || b0 + 1 >= m.size || b1 + 1 >= m.size || b2 + 1 >= m.size)
         return false;
-#pragma unroll 1
-    for (int n = 0; n < 8; ++n) {
-        const int vx = b0 + (n & 1), vy = b1 + ((n >> 1) & 1), vz = b2 + (n >> 2);
-        const int blk = lookup_block(m, c, vx, vy, vz);
-        if (blk < 0)
-            return false;
-        const int vi = (vx & 7) + 8 * (vy & 7) + 64 * (vz & 7);
-        float w;
-        load_voxel<S>(m, blk, vi, q.f[n], w);
-        if (!(w != 0.0f))
-            return false;
-        q.blk[n] = blk;
-        q.vi[n] = (short) vi;
-    }
+    if ((b0 != q.b0 || b1 != q.b1 || b2 != q.b2) && !tri_load<S>(m, q, b0, b1, b2))
+        return false;
     q.t = f3(bf.x - floorf(bf.x), bf.y - floorf(bf.y), bf.z - floorf(bf.z));
     const F3 t = q.t;
     const F3 tc = f3(1.0f - t.x, 1.0f - t.y, 1.0f - t.z);
@@ -87,8 +121,12 @@ __device__ bool diff_hit(const MapDevice& m, const RaycastParams& rp, BlockCache
     if (!(f_t >= 0.0f))
         return false;
     for (; t < t_far; t += stepsize) {
-        float f, w;
-        map_get_data<S>(m, c, p, f, w);
+        // the sample's voxel coordinates serve the lookup and the interpolation (see raycast_tsdf)
+        F3 vf;
+        const bool in_map = point_to_voxel_f(m, p, vf);
+        float f = 1.0f, w = 0.0f;
+        if (in_map)
+            fetch_voxel<S>(m, c, (int) vf.x, (int) vf.y, (int) vf.z, f, w);
         if (!(w != 0.0f)) {
             stepsize = largestep;
             p = add(p, mul(stepsize, d));
@@ -97,7 +135,7 @@ __device__ bool diff_hit(const MapDevice& m, const RaycastParams& rp, BlockCache
         f_tt = f;
         if (f_tt < 0.1f && f_tt >= -0.5f) {
             float fi;
-            if (field_interp<S>(m, c, p, fi))
+            if (field_interp_vf<S>(m, c, vf, fi))
                 f_tt = fi;
         }
         if (f_tt < 0.0f)
@@ -109,7 +147,8 @@ __device__ bool diff_hit(const MapDevice& m, const RaycastParams& rp, BlockCache
         return false;
     // bracket [t - stepsize, t] on the trilinear field
     float ta = t - stepsize, tb = t, fa, fb;
-    if (!tri_sample<S>(m, c, add(o, mul(d, ta)), q, fa) || !tri_sample<S>(m, c, add(o, mul(d, tb)), q, fb))
+    q.b0 = -1;
+    if (!tri_sample<S>(m, add(o, mul(d, ta)), q, fa) || !tri_sample<S>(m, add(o, mul(d, tb)), q, fb))
         return false;
     if (!(fa >= 0.0f && fb < 0.0f))
         return false;
@@ -119,7 +158,7 @@ __device__ bool diff_hit(const MapDevice& m, const RaycastParams& rp, BlockCache
     for (int it = 0; it < 40; ++it) {
         tm = (ta * fb - tb * fa) / (fb - fa);
         float fm;
-        if (!tri_sample<S>(m, c, add(o, mul(d, tm)), q, fm))
+        if (!tri_sample<S>(m, add(o, mul(d, tm)), q, fm))
             return false;
         if (fabsf(fm) < 1.0e-6f)
             break;
@@ -233,10 +272,10 @@ __global__ void __launch_bounds__(128) adjoint_kernel(MapDevice m, Pinhole s, Ra
                             const F3 t = q.t;
                             const F3 tc = f3(1.0f - t.x, 1.0f - t.y, 1.0f - t.z);
                             const float c0 = gd * k;
-#pragma unroll 1
+#pragma unroll
                             for (int n = 0; n < 8; ++n) {
                                 const float w = ((n & 1) ? t.x : tc.x) * (((n >> 1) & 1) ? t.y : tc.y) * ((n >> 2) ? t.z : tc.z);
-                                atomicAdd(&voxel_grad[(size_t) q.blk[n] * kBlockVoxels + q.vi[n]], c0 * w);
+                                atomicAdd(&voxel_grad[(size_t) q.blk[n] * kBlockVoxels + tri_voxel(q, n)], c0 * w);
                             }
                         }
                     }
