@@ -32,22 +32,36 @@ __global__ void raycast_prep_kernel(const float* pose12, RaycastParams host_p, R
     *out = p;
 }
 
-// TILE 0: each warp takes 8 x 4 pixels (a CTA 16 x 8); TILE 1: 16 x 2 (a CTA 32 x 4).
+// The pixel of a thread, TILE 0: each warp takes 8 x 4 pixels (a CTA 16 x 8); TILE 1: 16 x 2 (a CTA 32 x 4).
+template <int TILE>
+__device__ __forceinline__ bool raycast_pixel(const Pinhole& s, int& x, int& y)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int kWx = TILE == 0 ? 8 : 16, kWy = 32 / kWx; // warp tile
+    x = blockIdx.x * (2 * kWx) + (warp & 1) * kWx + (lane % kWx);
+    y = blockIdx.y * (2 * kWy) + (warp >> 1) * kWy + (lane / kWx);
+    return x < s.w && y < s.h;
+}
+
+// Single-res maps: the whole raycast. Multi-res maps: the points and scales, and in the normals' x whether
+// the pixel has a hit (1 or 0, the other components 0) for raycast_normal_kernel.
+//
+// The multi-res gradient is a kernel of its own because the code of both together does not stay in the
+// SM's instruction caches (9.3 stall cycles per issue went to instruction fetch, against 1.3 for the
+// single-res kernel): a 1280x960 pass of integration and raycast 501 us as one kernel, 441 as two. The
+// single-res kernel loses by the split (640x480, FP16: 149 against 151 us; 320x240: 68 against 70).
 template <int S, bool MR, int TILE>
-__global__ void __launch_bounds__(128, 9) raycast_kernel(MapDevice m, Pinhole s, const RaycastParams* __restrict__ P,
-                                                      float* __restrict__ pts, float* __restrict__ nrm,
-                                                      int8_t* __restrict__ scale)
+__global__ void __launch_bounds__(128, MR ? 10 : 9) raycast_kernel(MapDevice m, Pinhole s, const RaycastParams* __restrict__ P,
+                                                                float* __restrict__ pts, float* __restrict__ nrm,
+                                                                int8_t* __restrict__ scale)
 {
     grid_dep_wait();
     // per-thread scratch in shared memory (column threadIdx.x): the gradient's block table
-    __shared__ int sh_bt[8 * 128];
-    const RaycastParams rp = *P;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int kWx = TILE == 0 ? 8 : 16, kWy = 32 / kWx; // warp tile
-    const int x = blockIdx.x * (2 * kWx) + (warp & 1) * kWx + (lane % kWx);
-    const int y = blockIdx.y * (2 * kWy) + (warp >> 1) * kWy + (lane / kWx);
-    if (x >= s.w || y >= s.h)
+    __shared__ int sh_bt[MR ? 1 : 8 * 128];
+    int x, y;
+    if (!raycast_pixel<TILE>(s, x, y))
         return;
+    const RaycastParams rp = *P;
     const size_t idx = (size_t) x + (size_t) y * s.w;
     const F3 ray_S = back_project(s, (float) x, (float) y);
     const F3 nS = normalized(ray_S);
@@ -55,21 +69,21 @@ __global__ void __launch_bounds__(128, 9) raycast_kernel(MapDevice m, Pinhole s,
     const F3 origin = f3(rp.T_WS.t[0], rp.T_WS.t[1], rp.T_WS.t[2]);
     const float t_near = s.near_plane / nS.z;
     const float t_far = s.far_plane / nS.z;
-    BlockCache c{-1, -1, -1, -1};
+    RayCache<MR> c;
     F3 hit;
     F3 n = f3(0.0f, 0.0f, 0.0f);
     F3 p = f3(0.0f, 0.0f, 0.0f);
     int hit_scale = 0;
     if (raycast_tsdf<S, MR>(m, rp, c, origin, dir_W, t_near, t_far, hit, hit_scale)) {
         p = hit;
-        F3 g;
-        bool ok;
-        if constexpr (MR)
-            ok = mr_field_grad<S>(m, hit, g);
-        else
-            ok = field_grad_batched<S>(m, c, hit, g, sh_bt + threadIdx.x, 128);
-        if (ok)
-            n = normalized(g);
+        if constexpr (MR) {
+            n.x = 1.0f;
+        }
+        else {
+            F3 g;
+            if (field_grad_batched<S>(m, c.c, hit, g, sh_bt + threadIdx.x, 128))
+                n = normalized(g);
+        }
     }
     pts[3 * idx + 0] = p.x;
     pts[3 * idx + 1] = p.y;
@@ -81,32 +95,58 @@ __global__ void __launch_bounds__(128, 9) raycast_kernel(MapDevice m, Pinhole s,
         scale[idx] = (int8_t) hit_scale;
 }
 
-template <int S, bool MR>
-__global__ void field_query_kernel(MapDevice m, int n, const float* __restrict__ pts, float* __restrict__ out,
-                                   int* __restrict__ valid, int grad)
+// The normals at a multi-res raycast's hits.
+template <int S>
+__global__ void __launch_bounds__(128, 6) raycast_normal_kernel(MapDevice m, Pinhole s, const float* __restrict__ pts,
+                                                             float* __restrict__ nrm)
 {
+    grid_dep_wait();
+    __shared__ int sh_bt[8 * 128]; // the gradients' block tables, column threadIdx.x
+    int x, y;
+    if (!raycast_pixel<0>(s, x, y))
+        return;
+    const size_t idx = (size_t) x + (size_t) y * s.w;
+    if (nrm[3 * idx] == 0.0f)
+        return;
+    const F3 hit = f3(pts[3 * idx], pts[3 * idx + 1], pts[3 * idx + 2]);
+    MrCache c{-1, -1, -1, -1, -1};
+    F3 g, n = f3(0.0f, 0.0f, 0.0f);
+    if (mr_field_grad<S>(m, c, hit, g, sh_bt + threadIdx.x, 128))
+        n = normalized(g);
+    nrm[3 * idx + 0] = n.x;
+    nrm[3 * idx + 1] = n.y;
+    nrm[3 * idx + 2] = n.z;
+}
+
+// The batched field queries, a thread per point. A gradient's 32 samples are in flight together, as in
+// the raycast.
+template <int S, bool MR, bool GRAD>
+__global__ void __launch_bounds__(128) field_query_kernel(MapDevice m, int n, const float* __restrict__ pts,
+                                                          float* __restrict__ out, int* __restrict__ valid)
+{
+    __shared__ int sh_bt[GRAD ? 8 * 128 : 1];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
-    const F3 p = f3(pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]);
-    BlockCache c{-1, -1, -1, -1};
+    const F3 p = f3(pts[3 * (size_t) i], pts[3 * (size_t) i + 1], pts[3 * (size_t) i + 2]);
+    RayCache<MR> c;
     bool ok;
-    if (grad) {
+    if constexpr (GRAD) {
         F3 g = f3(0.0f, 0.0f, 0.0f);
         if constexpr (MR)
-            ok = mr_field_grad<S>(m, p, g);
+            ok = mr_field_grad<S>(m, c.c, p, g, sh_bt + threadIdx.x, 128);
         else
-            ok = field_grad<S>(m, c, p, g);
-        out[3 * i] = ok ? g.x : 0.0f;
-        out[3 * i + 1] = ok ? g.y : 0.0f;
-        out[3 * i + 2] = ok ? g.z : 0.0f;
+            ok = field_grad_batched<S>(m, c.c, p, g, sh_bt + threadIdx.x, 128);
+        out[3 * (size_t) i] = ok ? g.x : 0.0f;
+        out[3 * (size_t) i + 1] = ok ? g.y : 0.0f;
+        out[3 * (size_t) i + 2] = ok ? g.z : 0.0f;
     }
     else {
         float v = 0.0f;
         if constexpr (MR)
             ok = mr_field_interp<S>(m, p, v, nullptr);
         else
-            ok = field_interp<S>(m, c, p, v);
+            ok = field_interp<S>(m, c.c, p, v);
         out[i] = ok ? v : 0.0f;
     }
     if (valid)
@@ -134,6 +174,8 @@ se_gpu_status enqueue_raycast(const se_gpu_map* map, const se_gpu_pinhole& senso
     rp.scaling = (float) m.size * m.res;
     rp.eps = std::exp2((float) (-std::log2((double) m.size)));
     rp.min_scale = 23 - m.log2_bps;
+    // (a launch of its own also keeps the raycast's CTAs off the SMs until the update is done: scheduled
+    // in its tail they pile up on the SMs that are free first, 320x240 67 -> 77 us)
     launch_chained(raycast_prep_kernel, 1, 1, stream, T_WS_host16 ? nullptr : pose12_dev, rp, map->rparams);
     const int tile = map->tiles.raycast_tile;
     const dim3 grid = tile == 0 ? dim3((s.w + 15) / 16, (s.h + 7) / 8) : dim3((s.w + 31) / 32, (s.h + 3) / 4);
@@ -149,6 +191,9 @@ se_gpu_status enqueue_raycast(const se_gpu_map* map, const se_gpu_pinhole& senso
         else                                                                                                        \
             launch_chained(raycast_kernel<S_, MR_, 1>, grid, 128, stream, m, s, map->rparams, pts_dev, nrm_dev,     \
                            scale_dev);                                                                              \
+        if (MR_)                                                                                                    \
+            launch_chained(raycast_normal_kernel<S_>, dim3((s.w + 15) / 16, (s.h + 7) / 8), 128, stream, m, s,      \
+                           pts_dev, nrm_dev);                                                                       \
     } while (0)
     if (m.storage == SE_GPU_STORAGE_F32 && !mr)
         SE_RAYCAST_LAUNCH(SE_GPU_STORAGE_F32, false);
@@ -197,14 +242,22 @@ static se_gpu_status field_query(const se_gpu_map* map, int64_t n, const float* 
     cudaStream_t stream = (cudaStream_t) stream_p;
     const unsigned blocks = (unsigned) ((n + 127) / 128);
     const bool mr = map->dev.res_type == SE_GPU_RES_MULTI;
+#define SE_QUERY_LAUNCH(S_, MR_)                                                                                     \
+    do {                                                                                                            \
+        if (grad)                                                                                                   \
+            field_query_kernel<S_, MR_, true><<<blocks, 128, 0, stream>>>(map->dev, (int) n, pts, out, valid);       \
+        else                                                                                                        \
+            field_query_kernel<S_, MR_, false><<<blocks, 128, 0, stream>>>(map->dev, (int) n, pts, out, valid);      \
+    } while (0)
     if (map->dev.storage == SE_GPU_STORAGE_F32 && !mr)
-        field_query_kernel<SE_GPU_STORAGE_F32, false><<<blocks, 128, 0, stream>>>(map->dev, (int) n, pts, out, valid, grad);
+        SE_QUERY_LAUNCH(SE_GPU_STORAGE_F32, false);
     else if (!mr)
-        field_query_kernel<SE_GPU_STORAGE_F16, false><<<blocks, 128, 0, stream>>>(map->dev, (int) n, pts, out, valid, grad);
+        SE_QUERY_LAUNCH(SE_GPU_STORAGE_F16, false);
     else if (map->dev.storage == SE_GPU_STORAGE_F32)
-        field_query_kernel<SE_GPU_STORAGE_F32, true><<<blocks, 128, 0, stream>>>(map->dev, (int) n, pts, out, valid, grad);
+        SE_QUERY_LAUNCH(SE_GPU_STORAGE_F32, true);
     else
-        field_query_kernel<SE_GPU_STORAGE_F16, true><<<blocks, 128, 0, stream>>>(map->dev, (int) n, pts, out, valid, grad);
+        SE_QUERY_LAUNCH(SE_GPU_STORAGE_F16, true);
+#undef SE_QUERY_LAUNCH
     SE_CUDA_TRY(cudaGetLastError());
     return SE_GPU_OK;
 }
