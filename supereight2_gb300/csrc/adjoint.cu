@@ -107,7 +107,7 @@ __device__ bool diff_hit(const MapDevice& m, const RaycastParams& rp, BlockCache
                          float t_far, float& t_star, Tri& q)
 {
     float t_min, t_max;
-    first_block(m, rp, o, d, t_near, t_far, t_min, t_max);
+    first_block(m, rp, d, t_near, t_far, t_min, t_max);
     if (t_min <= 0.0f || !(t_near < t_max))
         return false;
     const float step = m.res;
@@ -135,7 +135,7 @@ __device__ bool diff_hit(const MapDevice& m, const RaycastParams& rp, BlockCache
         f_tt = f;
         if (f_tt < 0.1f && f_tt >= -0.5f) {
             float fi;
-            if (field_interp_vf<S>(m, c, vf, fi))
+            if (field_interp_vf<S>(m, vf, fi))
                 f_tt = fi;
         }
         if (f_tt < 0.0f)
@@ -303,6 +303,7 @@ static RaycastParams host_raycast_params(const MapDevice& m, const float* T_WS)
     rp.scaling = (float) m.size * m.res;
     rp.eps = std::exp2((float) (-std::log2((double) m.size)));
     rp.min_scale = 23 - m.log2_bps;
+    set_raycast_origin(m, rp);
     return rp;
 }
 

@@ -23,12 +23,13 @@
 
 namespace se_gpu {
 
-__global__ void raycast_prep_kernel(const float* pose12, RaycastParams host_p, RaycastParams* out)
+__global__ void raycast_prep_kernel(const float* pose12, RaycastParams host_p, MapDevice m, RaycastParams* out)
 {
     grid_dep_wait();
     RaycastParams p = host_p;
     if (pose12 != nullptr)
         p.T_WS = tf_from12(pose12);
+    set_raycast_origin(m, p);
     *out = p;
 }
 
@@ -146,7 +147,7 @@ __global__ void __launch_bounds__(128) field_query_kernel(MapDevice m, int n, co
         if constexpr (MR)
             ok = mr_field_interp<S>(m, p, v, nullptr);
         else
-            ok = field_interp<S>(m, c.c, p, v);
+            ok = field_interp<S>(m, p, v);
         out[i] = ok ? v : 0.0f;
     }
     if (valid)
@@ -176,7 +177,7 @@ se_gpu_status enqueue_raycast(const se_gpu_map* map, const se_gpu_pinhole& senso
     rp.min_scale = 23 - m.log2_bps;
     // (a launch of its own also keeps the raycast's CTAs off the SMs until the update is done: scheduled
     // in its tail they pile up on the SMs that are free first, 320x240 67 -> 77 us)
-    launch_chained(raycast_prep_kernel, 1, 1, stream, T_WS_host16 ? nullptr : pose12_dev, rp, map->rparams);
+    launch_chained(raycast_prep_kernel, 1, 1, stream, T_WS_host16 ? nullptr : pose12_dev, rp, m, map->rparams);
     const int tile = map->tiles.raycast_tile;
     const dim3 grid = tile == 0 ? dim3((s.w + 15) / 16, (s.h + 7) / 8) : dim3((s.w + 31) / 32, (s.h + 3) / 4);
     ProfScope ps(kProfRaycast, stream);

@@ -42,21 +42,19 @@ constexpr int kDdaTopLevel = 2;
 // a cell edge, where the reference decides a tie at a coarser level than this walk: 0 of 921,600
 // rays of three 640x480 frames of the 1 cm benchmark map (and 1-2 per frame when starting at
 // levels 0 or 1).
-static __device__ bool first_block(const MapDevice& m, const RaycastParams& rp, F3 o_W, F3 d_W, float near_p,
-                                   float far_p, float& tcmin, float& tmax)
+static __device__ bool first_block(const MapDevice& m, const RaycastParams& rp, F3 d_W, float near_p, float far_p,
+                                   float& tcmin, float& tmax)
 {
     float d[3] = {d_W.x, d_W.y, d_W.z};
 #pragma unroll
     for (int a = 0; a < 3; ++a)
         if (fabsf(d[a]) < rp.eps)
             d[a] = copysignf(rp.eps, d[a]);
-    const F3 o_M = apply(m.T_MW, o_W);
-    const float ov[3] = {o_M.x / m.res, o_M.y / m.res, o_M.z / m.res};
     float t_coef[3], t_bias[3];
     bool flip[3]; // the axes the unit cube mirrors (the ray runs towards larger coordinates)
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        const float o = ov[a] / (float) m.size + 1.0f;
+        const float o = rp.origin[a];
         t_coef[a] = -1.0f * (1.0f / fabsf(d[a]));
         t_bias[a] = t_coef[a] * o;
         flip[a] = d[a] > 0.0f;
@@ -224,61 +222,51 @@ __device__ __forceinline__ void map_get_data(const MapDevice& m, BlockCache& c, 
     fetch_voxel<S>(m, c, vx, vy, vz, t, w);
 }
 
-// visitor::getInterp single-res: any unallocated block or invalid voxel gives nullopt.
+// visitor::getInterp single-res from the point's voxel coordinates (point_to_voxel_f, inside the map): any
+// unallocated block or invalid voxel gives nullopt.
 template <int S>
-__device__ bool field_interp_vf(const MapDevice& m, BlockCache& c, F3 vf, float& out);
-
-template <int S>
-__device__ bool field_interp(const MapDevice& m, BlockCache& c, F3 p_W, float& out)
-{
-    F3 vf;
-    if (!point_to_voxel_f(m, p_W, vf))
-        return false;
-    return field_interp_vf<S>(m, c, vf, out);
-}
-
-// field_interp from the point's voxel coordinates (point_to_voxel_f, inside the map).
-template <int S>
-__device__ bool field_interp_vf(const MapDevice& m, BlockCache& c, F3 vf, float& out)
+__device__ bool field_interp_vf(const MapDevice& m, F3 vf, float& out)
 {
     const F3 bf = f3(vf.x - 0.5f, vf.y - 0.5f, vf.z - 0.5f);
     const int b0 = (int) bf.x, b1 = (int) bf.y, b2 = (int) bf.z;
     if (b0 < 0 || b1 < 0 || b2 < 0 || b0 + 1 >= m.size || b1 + 1 >= m.size || b2 + 1 >= m.size)
         return false;
+    // The blocks of the 2 x 2 x 2 corners, then the voxels, each 8 loads in flight together. One path for
+    // cells inside a block and across blocks: a third of the cells are of the second kind, so nearly every
+    // warp ran both (640x480 raycast and integration, FP16: 148 us with the corners of a cell across blocks
+    // one after another, 138.3 with these loads for it, 137.6 so).
     float f[8];
-    if ((b0 & 7) != 7 && (b1 & 7) != 7 && (b2 & 7) != 7) {
-        // the 8 neighbours share one block
-        const int blk = lookup_block(m, c, b0, b1, b2);
-        if (blk < 0)
-            return false;
-        const int base = (b0 & 7) + 8 * (b1 & 7) + 64 * (b2 & 7);
-        bool ok = true;
+    int blk[8];
+    const int s1 = m.log2_bps, s2 = 2 * m.log2_bps;
+    const uint32_t X0 = b0 >> 3, X1 = (b0 + 1) >> 3, Y0 = (uint32_t) (b1 >> 3) << s1, Y1 = (uint32_t) ((b1 + 1) >> 3) << s1;
+    const uint32_t Z0 = (uint32_t) (b2 >> 3) << s2, Z1 = (uint32_t) ((b2 + 1) >> 3) << s2;
+    bool ok = true;
 #pragma unroll
-        for (int n = 0; n < 8; ++n) {
-            float w;
-            load_voxel<S>(m, blk, base + (n & 1) + 8 * ((n >> 1) & 1) + 64 * (n >> 2), f[n], w);
-            ok = ok && (w != 0.0f);
-        }
-        if (!ok)
-            return false;
+    for (int n = 0; n < 8; ++n) {
+        blk[n] = __ldg(&m.block_index[((n & 1) ? X1 : X0) | ((n & 2) ? Y1 : Y0) | ((n & 4) ? Z1 : Z0)]);
+        ok = ok && blk[n] >= 0;
     }
-    else {
-        bool ok = true;
-#pragma unroll 1
-        for (int n = 0; n < 8; ++n) {
-            float w;
-            if (!fetch_voxel<S>(m, c, b0 + (n & 1), b1 + ((n >> 1) & 1), b2 + ((n >> 2) & 1), f[n], w))
-                return false; // an unallocated block fails before any validity test
-            ok = ok && (w != 0.0f);
-        }
-        if (!ok)
-            return false;
-    }
+    if (!ok)
+        return false;
+    const int x0 = b0 & 7, y0 = 8 * (b1 & 7), z0 = 64 * (b2 & 7);
+    const int x1 = (b0 + 1) & 7, y1 = 8 * ((b1 + 1) & 7), z1 = 64 * ((b2 + 1) & 7);
+#pragma unroll
+    for (int n = 0; n < 8; ++n)
+        ok = load_tsdf<S>(m, blk[n], ((n & 1) ? x1 : x0) + ((n & 2) ? y1 : y0) + ((n & 4) ? z1 : z0), f[n]) && ok;
+    if (!ok)
+        return false;
     const F3 t = f3(bf.x - floorf(bf.x), bf.y - floorf(bf.y), bf.z - floorf(bf.z));
     const F3 tc = f3(1.0f - t.x, 1.0f - t.y, 1.0f - t.z);
     out = ((f[0] * tc.x + f[1] * t.x) * tc.y + (f[2] * tc.x + f[3] * t.x) * t.y) * tc.z
         + ((f[4] * tc.x + f[5] * t.x) * tc.y + (f[6] * tc.x + f[7] * t.x) * t.y) * t.z;
     return true;
+}
+
+template <int S>
+__device__ bool field_interp(const MapDevice& m, F3 p_W, float& out)
+{
+    F3 vf;
+    return point_to_voxel_f(m, p_W, vf) && field_interp_vf<S>(m, vf, out);
 }
 
 // visitor::getFieldGrad single-res with Map::getFieldGrad's division by the resolution, its 32 samples (grad_sel)
@@ -329,10 +317,8 @@ __device__ bool field_grad_batched(const MapDevice& m, BlockCache& c, F3 p_W, F3
         const int code = grad_sel(i);
         const int x = sel[0][code & 3], y = sel[1][(code >> 2) & 3], z = sel[2][(code >> 4) & 3];
         const int b = bt[(((x >> 3) - lo[0]) | (((y >> 3) - lo[1]) << 1) | (((z >> 3) - lo[2]) << 2)) * bs];
-        float t = 1.0f, w = 0.0f;
-        if (b >= 0)
-            load_voxel<S>(m, b, (x & 7) + 8 * (y & 7) + 64 * (z & 7), t, w);
-        ok = ok && (w != 0.0f);
+        float t = 1.0f;
+        ok = b >= 0 && load_tsdf<S>(m, b, (x & 7) + 8 * (y & 7) + 64 * (z & 7), t) && ok;
         v[i] = t;
     }
     if (!ok)
@@ -396,7 +382,7 @@ __device__ bool raycast_tsdf(const MapDevice& m, const RaycastParams& rp, RayCac
 {
     int scale_tt = 0;
     float t_min, t_max;
-    first_block(m, rp, o, d, t_near, t_far, t_min, t_max);
+    first_block(m, rp, d, t_near, t_far, t_min, t_max);
     if (t_min <= 0.0f)
         return false;
     const float step = m.res;
@@ -445,7 +431,7 @@ __device__ bool raycast_tsdf(const MapDevice& m, const RaycastParams& rp, RayCac
             if constexpr (MR)
                 ok = mr_interp<S>(m, rc.c, vf, 0, fi, &scale_tt);
             else
-                ok = field_interp_vf<S>(m, rc.c, vf, fi);
+                ok = field_interp_vf<S>(m, vf, fi);
             if (ok)
                 f_tt = fi;
         }
