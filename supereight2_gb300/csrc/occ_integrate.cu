@@ -79,6 +79,40 @@ __device__ __forceinline__ int push(int* list, int* count, int cap, int v, int* 
     return k;
 }
 
+// Stages of a few warps' work a map run as one cluster of CTAs for each map: the cluster's CTAs are resident
+// together, so its barrier always ends and the launch may be chained like any other.
+constexpr int kOccCluster = 8, kOccClusterThreads = 512;
+constexpr int kOccTopCarve = 2;     // the carver's depths in occ_carve_top_kernel
+constexpr int kOccTopPropagate = 4; // the propagation's depths in occ_propagate_top_kernel
+
+__device__ __forceinline__ void occ_cluster_sync()
+{
+    __syncwarp();
+    __threadfence();
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    __threadfence();
+    __syncwarp();
+}
+
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_clusters(void (*kernel)(KArgs...), int maps, cudaStream_t stream, Args... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(maps * kOccCluster);
+    cfg.blockDim = dim3(kOccClusterThreads);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = kOccCluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 // -------------------------------------------------------------------------- begin --
 
 __device__ __forceinline__ void occ_begin(const OccLaunch& L, const OccStep& step, int j)
@@ -104,12 +138,18 @@ __device__ __forceinline__ void occ_begin(const OccLaunch& L, const OccStep& ste
 // replays unchanged).
 __global__ void occ_begin_kernel(const OccLaunch* __restrict__ Lp, const __grid_constant__ OccStep step)
 {
+    grid_dep_wait();
     occ_begin(*Lp, step, blockIdx.x);
 }
 __global__ void occ_begin_dev_kernel(const OccLaunch* __restrict__ Lp, const OccStep* __restrict__ step)
 {
+    grid_dep_wait();
     occ_begin(*Lp, *step, blockIdx.x);
 }
+
+// 0.95 * -100 of the reference's tests, which is -95 in double.
+constexpr float kOccFreeField = -95.0f;
+static_assert(0.95 * -100.0 == (double) kOccFreeField);
 
 // ------------------------------------------------------------------ per-pixel inputs --
 
@@ -134,6 +174,7 @@ __device__ __forceinline__ void occ_pixel(const OccLaunch& L, int j, int i)
 
 __global__ void occ_pixels_kernel(const OccLaunch* __restrict__ Lp)
 {
+    grid_dep_wait();
     const OccLaunch& L = *Lp;
     const int npx = L.sensor.w * L.sensor.h;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -216,6 +257,7 @@ __device__ __forceinline__ void occ_pool_pixel(const OccLaunch& L, int level, in
 
 __global__ void occ_pool_level_kernel(const OccLaunch* __restrict__ Lp, int level)
 {
+    grid_dep_wait();
     const OccLaunch& L = *Lp;
     const int npx = L.sensor.w * L.sensor.h;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -271,10 +313,9 @@ __device__ PoolPair pool_bounding_box(const float4* __restrict__ pool_d, const f
 {
     const int min_side = min(u_max - u_min, v_max - v_min);
     const int half = min_side / 2;
-    // log2(0) = -inf: the reference's clamps turn it into level 0
-    int lc = INT_MIN;
-    if (half > 0)
-        lc = (int) ceil(log2((double) half));
+    // ceil(log2(half)) in integers (in FP64 it was a good part of an octant's time); log2(0) = -inf, which
+    // the reference's clamps turn into level 0
+    const int lc = half > 0 ? 32 - __clz(half - 1) : INT_MIN;
     const int level = max(0, min(max_level, lc));
     const int s = level > 0 ? 1 << max(level - 1, 0) : 0;
     const int step = 2 * s + 1;
@@ -542,14 +583,6 @@ __device__ void occ_root(const OccLaunch& L, int j, int lane)
     m.counters[kOccFrontierN + 1] = n;
 }
 
-__global__ void occ_root_kernel(const OccLaunch* __restrict__ Lp)
-{
-    const OccLaunch& L = *Lp;
-    if (blockIdx.x >= L.n || threadIdx.x >= 32)
-        return;
-    occ_root(L, blockIdx.x, threadIdx.x & 31);
-}
-
 // cameraInNode with pointToVoxel<Safe::On> (volume_carver_impl.hpp:83-98)
 __device__ __forceinline__ bool camera_in_node(const OccDevice& m, const Tf& T_WS, int cx, int cy, int cz, int size)
 {
@@ -564,6 +597,13 @@ __device__ __forceinline__ bool camera_in_node(const OccDevice& m, const Tf& T_W
         && vz >= (float) cz && vz <= (float) (cz + size);
 }
 
+// z > 1.25 x without FP64: p = RN(1.25 x), e = 1.25 x - p exact; no float lies between p and p + e.
+__device__ __forceinline__ bool above_scaled(float z, float x)
+{
+    const float p = 1.25f * x;
+    return z > p || (z == p && fmaf(1.25f, x, -p) < 0.0f);
+}
+
 // computeVariance (volume_carver_impl.hpp:100-126): 0 Constant, 1 Gradient, 2 Undefined
 __device__ __forceinline__ int compute_variance(const OccJob& J, float d_min, float d_max, float n_min, float n_max,
                                                 float std_max)
@@ -573,9 +613,10 @@ __device__ __forceinline__ int compute_variance(const OccJob& J, float d_min, fl
     const float tv = J.m.cfg.k_tau * d_max;
     const float tau_max = tv < J.tau_min ? J.tau_min : (J.tau_max < tv ? J.tau_max : tv);
     const float three_sigma_min = 3.0f * std_max;
-    if ((double) z_diff_min > 1.25 * (double) tau_max)
+    // the reference's comparisons are in double, where 1.25 x is exact
+    if (above_scaled(z_diff_min, tau_max))
         return 2;
-    if ((double) z_diff_max < -1.25 * (double) three_sigma_min)
+    if (above_scaled(-z_diff_max, three_sigma_min))
         return 0;
     return 1;
 }
@@ -623,7 +664,7 @@ __device__ __forceinline__ bool carve_pooled(const OccLaunch& L, const OccJob& J
     var = compute_variance(J, pp.min, pp.max, n_min, n_max, q.sigma_max);
     if (var != 1) {
         const OccD cd = octant_max_data(J.m, slot);
-        if (cd.observed && (double) occ_field(cd) <= 0.95 * -100.0)
+        if (cd.observed && occ_field(cd) <= kOccFreeField)
             return false;
     }
     if (pp.crossing == 1)
@@ -742,81 +783,106 @@ __device__ bool carve_lidar(const OccLaunch& L, const OccJob& J, const OccDyn& D
                         should_split, var, projects_inside, lane);
 }
 
-// One depth of the VolumeCarver over every map's frontier at that depth, one warp per octant;
-// lane 0 lists the octant or allocates and queues its children.
+// The VolumeCarver on one octant of a map's frontier at one depth, by a warp; lane 0 lists the octant or
+// allocates and queues its children.
+__device__ __forceinline__ void occ_carve_octant(const OccLaunch& L, const OccJob& J, int depth, int at, int lane)
+{
+    const OccDevice& m = J.m;
+    const OccDyn& D = *J.dyn;
+    int* err = &m.counters[kOccError];
+    const int slot = J.frontier[depth & 1][at];
+    const bool is_block = slot_is_block(slot);
+    int cx, cy, cz, size;
+    if (is_block) {
+        const int b = slot_block(slot);
+        cx = m.block_coord[3 * b];
+        cy = m.block_coord[3 * b + 1];
+        cz = m.block_coord[3 * b + 2];
+        size = 8;
+    }
+    else {
+        const int4 nc = m.node_coord[slot];
+        cx = nc.x;
+        cy = nc.y;
+        cz = nc.z;
+        size = nc.w;
+    }
+    bool should_split = false, projects_inside = false;
+    int var = 1; // Gradient
+    const float max_depth_value = J.max_value[1];
+    const bool keep = L.sensor.lidar
+        ? carve_lidar(L, J, D, slot, cx, cy, cz, size, max_depth_value, should_split, var, projects_inside, lane)
+        : carve_pinhole(L, J, D, slot, cx, cy, cz, size, max_depth_value, should_split, var, projects_inside,
+                        lane);
+    if (keep && !is_block && should_split) {
+        occ_allocate_children_warp(m, slot, lane);
+        // queue the children: one atomic for all of them, lane i writes child i
+        const int ch = lane < 8 ? m.node_child[8 * (size_t) slot + lane] : -1;
+        const unsigned mask = __ballot_sync(0xffffffffu, ch != -1); // -1 only when a pool ran out
+        int base = 0;
+        if (lane == 0 && mask)
+            base = atomicAdd(&m.counters[kOccFrontierN + depth + 1], __popc(mask));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (ch != -1) {
+            const int k = base + __popc(mask & ((1u << lane) - 1u));
+            if (k < m.node_capacity + m.block_capacity)
+                J.frontier[(depth + 1) & 1][k] = ch;
+            else
+                atomicOr(err, kOccErrList);
+        }
+    }
+    else if (keep && lane == 0) {
+        if (is_block) {
+            const int k = push(J.block_list, &m.counters[kOccBlockListN], m.block_capacity, slot_block(slot), err);
+            if (k < m.block_capacity) {
+                J.block_var[k] = var;
+                J.block_inside[k] = projects_inside ? 1 : 0;
+            }
+        }
+        else if (var == 0) {
+            push(J.node_list, &m.counters[kOccNodeListN], m.node_capacity, slot, err);
+        }
+    }
+    __syncwarp();
+}
+
+// One depth of the VolumeCarver over every map's frontier at that depth, one warp per octant.
 __device__ void occ_carve_stage(const OccLaunch& L, int depth, int bid, int nbid)
 {
     __shared__ int pre[kOccMaxBatch + 1];
     const int total = batch_prefix(L, pre, [depth](const OccJob& J) {
         return clamp_count(J.m.counters[kOccFrontierN + depth], J.m.node_capacity + J.m.block_capacity);
     });
-    const int lane = threadIdx.x & 31;
     const int n_warps = (nbid * blockDim.x) >> 5;
     for (int idx = (bid * blockDim.x + threadIdx.x) >> 5; idx < total; idx += n_warps) {
         const int j = batch_find(pre, L.n, idx);
-        const OccJob& J = L.job[j];
-        const OccDevice& m = J.m;
-        const OccDyn& D = *J.dyn;
-        int* err = &m.counters[kOccError];
-        const int slot = J.frontier[depth & 1][idx - pre[j]];
-        const bool is_block = slot_is_block(slot);
-        int cx, cy, cz, size;
-        if (is_block) {
-            const int b = slot_block(slot);
-            cx = m.block_coord[3 * b];
-            cy = m.block_coord[3 * b + 1];
-            cz = m.block_coord[3 * b + 2];
-            size = 8;
-        }
-        else {
-            const int4 nc = m.node_coord[slot];
-            cx = nc.x;
-            cy = nc.y;
-            cz = nc.z;
-            size = nc.w;
-        }
-        bool should_split = false, projects_inside = false;
-        int var = 1; // Gradient
-        const float max_depth_value = J.max_value[1];
-        const bool keep = L.sensor.lidar
-            ? carve_lidar(L, J, D, slot, cx, cy, cz, size, max_depth_value, should_split, var, projects_inside, lane)
-            : carve_pinhole(L, J, D, slot, cx, cy, cz, size, max_depth_value, should_split, var, projects_inside,
-                            lane);
-        if (keep && !is_block && should_split) {
-            occ_allocate_children_warp(m, slot, lane);
-            // queue the children: one atomic for all of them, lane i writes child i
-            const int ch = lane < 8 ? m.node_child[8 * (size_t) slot + lane] : -1;
-            const unsigned mask = __ballot_sync(0xffffffffu, ch != -1); // -1 only when a pool ran out
-            int base = 0;
-            if (lane == 0 && mask)
-                base = atomicAdd(&m.counters[kOccFrontierN + depth + 1], __popc(mask));
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (ch != -1) {
-                const int k = base + __popc(mask & ((1u << lane) - 1u));
-                if (k < m.node_capacity + m.block_capacity)
-                    J.frontier[(depth + 1) & 1][k] = ch;
-                else
-                    atomicOr(err, kOccErrList);
-            }
-        }
-        else if (keep && lane == 0) {
-            if (is_block) {
-                const int k = push(J.block_list, &m.counters[kOccBlockListN], m.block_capacity, slot_block(slot), err);
-                if (k < m.block_capacity) {
-                    J.block_var[k] = var;
-                    J.block_inside[k] = projects_inside ? 1 : 0;
-                }
-            }
-            else if (var == 0) {
-                push(J.node_list, &m.counters[kOccNodeListN], m.node_capacity, slot, err);
-            }
-        }
-        __syncwarp();
+        occ_carve_octant(L, L.job[j], depth, idx - pre[j], threadIdx.x & 31);
+    }
+}
+
+// occ_root and the VolumeCarver's first depths (up to 8^d octants at depth d), a cluster of CTAs for each
+// map: see occ_propagate_top_kernel.
+__global__ void __launch_bounds__(kOccClusterThreads) occ_carve_top_kernel(const OccLaunch* __restrict__ Lp, int depths)
+{
+    grid_dep_wait();
+    const OccLaunch& L = *Lp;
+    const int j = blockIdx.x / kOccCluster;
+    const OccJob& J = L.job[j];
+    const int lane = threadIdx.x & 31;
+    const int warp = (blockIdx.x % kOccCluster) * (kOccClusterThreads / 32) + (threadIdx.x >> 5);
+    if (warp == 0)
+        occ_root(L, j, lane);
+    for (int d = 1; d <= depths; ++d) {
+        occ_cluster_sync();
+        const int total = clamp_count(J.m.counters[kOccFrontierN + d], J.m.node_capacity + J.m.block_capacity);
+        for (int i = warp; i < total; i += kOccCluster * (kOccClusterThreads / 32))
+            occ_carve_octant(L, J, d, i, lane);
     }
 }
 
 __global__ void __launch_bounds__(128) occ_carve_kernel(const OccLaunch* __restrict__ Lp, int depth)
 {
+    grid_dep_wait();
     occ_carve_stage(*Lp, depth, blockIdx.x, gridDim.x);
 }
 
@@ -867,6 +933,7 @@ __device__ void occ_nodes_stage(const OccLaunch& L, int bid, int nbid)
 
 __global__ void occ_nodes_kernel(const OccLaunch* __restrict__ Lp)
 {
+    grid_dep_wait();
     occ_nodes_stage(*Lp, blockIdx.x, gridDim.x);
 }
 
@@ -923,6 +990,7 @@ __device__ void occ_free_nodes_stage(const OccLaunch& L, int level, int bid, int
 
 __global__ void occ_free_nodes_kernel(const OccLaunch* __restrict__ Lp, int level)
 {
+    grid_dep_wait();
     occ_free_nodes_stage(*Lp, level, blockIdx.x, gridDim.x);
 }
 
@@ -958,22 +1026,16 @@ __device__ int pinhole_integration_scale(const Pinhole& s, float z, float res, i
 
 // OusterLidar::computeIntegrationScaleImpl (ouster_lidar.cpp:107-146): the chord between
 // neighbouring rays, 2 r tan(min_ray_angle / 2), against the voxel diagonal sqrt(3) res; the
-// hysteresis moves the point 0.25 m along its ray.
-__device__ int lidar_integration_scale(const Lidar& ld, F3 c, float res, int last_scale, int min_scale)
+// hysteresis moves the point 0.25 m along its ray. The reference divides in double; bounds (see
+// lidar_scale_bound) are the least chords whose rounded ratios reach 1.5, 3 and 6.
+__device__ int lidar_integration_scale(const Lidar& ld, F3 c, const float* bounds, int last_scale, int min_scale)
 {
     for (int pass = 0; pass < 2; ++pass) {
         const float dist = norm(c);
         const float pixel_dim = 2.0f * dist * ld.tan_half_min_angle;
-        const float pv = (float) ((double) pixel_dim / (sqrt(3.0) * (double) res));
         int scale = 0;
-        if (pv >= 1.5f) {
-            scale = 1;
-            if (pv >= 3.0f) {
-                scale = 2;
-                if (pv >= 6.0f)
-                    scale = 3;
-            }
-        }
+        if (pixel_dim >= bounds[0])
+            scale = pixel_dim >= bounds[1] ? (pixel_dim >= bounds[2] ? 3 : 2) : 1;
         if (pass == 0 && min_scale != -1 && scale != last_scale) {
             const F3 n = normalized(c);
             c = scale > last_scale ? sub(c, mul(0.25f, n)) : add(c, mul(0.25f, n));
@@ -1229,13 +1291,13 @@ __device__ void occ_update_block_data(const OccLaunch& L, const OccJob& J, const
     __syncwarp();
 }
 
-__device__ __forceinline__ int occ_recommended_scale(const OccLaunch& L, const OccDevice& m, int b,
+__device__ __forceinline__ int occ_recommended_scale(const OccLaunch& L, const OccDevice& m, const float* lidar_bounds, int b,
                                                      const OccBlockState& st, F3 centre_C, bool free_min,
                                                      int& last_scale)
 {
     last_scale = (st.min_scale == -1) ? 0 : st.current_scale;
     const int computed = L.sensor.lidar
-        ? lidar_integration_scale(L.sensor.L, centre_C, m.res, last_scale, st.min_scale)
+        ? lidar_integration_scale(L.sensor.L, centre_C, lidar_bounds, last_scale, st.min_scale)
         : pinhole_integration_scale(L.sensor.s, centre_C.z, m.res, last_scale, st.min_scale);
     const OccD mx = blk_max(m, b, st.finest, kOccMaxScale)[0];
     const int min_integr = (free_min && (st.min_scale == -1 || (double) mx.occ < 0.95 * (double) m.cfg.log_odd_min))
@@ -1257,7 +1319,7 @@ __device__ void occ_process_block(const OccLaunch& L, const OccJob& J, int b, bo
                                                        ((float) m.block_coord[3 * b + 1] + off) * m.res,
                                                        ((float) m.block_coord[3 * b + 2] + off) * m.res)));
     int last_scale;
-    const int rec = occ_recommended_scale(L, m, b, st, centre_C, free ? true : low_var, last_scale);
+    const int rec = occ_recommended_scale(L, m, J.lidar_bounds, b, st, centre_C, free ? true : low_var, last_scale);
     int integration_scale = last_scale;
     bool done = false;
     if (st.min_scale == -1) {
@@ -1336,78 +1398,13 @@ __device__ void occ_process_block(const OccLaunch& L, const OccJob& J, int b, bo
     __syncwarp();
 }
 
-// freeBlock on the freed blocks and updateBlock on the carver's blocks (disjoint: the carver
-// does not descend below a free-space node), one warp per block, all maps.
-__device__ void occ_blocks_stage(const OccLaunch& L, int bid, int nbid)
-{
-    __shared__ int pre[kOccMaxBatch + 1];
-    const int total = batch_prefix(L, pre, [](const OccJob& J) {
-        return clamp_count(J.m.counters[kOccFreedN], J.m.block_capacity)
-            + clamp_count(J.m.counters[kOccBlockListN], J.m.block_capacity);
-    });
-    const int lane = threadIdx.x & 31;
-    const int n_warps = (nbid * blockDim.x) >> 5;
-    for (int idx = (bid * blockDim.x + threadIdx.x) >> 5; idx < total; idx += n_warps) {
-        const int j = batch_find(pre, L.n, idx);
-        const OccJob& J = L.job[j];
-        const int n_freed = clamp_count(J.m.counters[kOccFreedN], J.m.block_capacity);
-        const int i = idx - pre[j];
-        if (i < n_freed)
-            occ_process_block(L, J, J.freed[i], true, true, true, lane);
-        else
-            occ_process_block(L, J, J.block_list[i - n_freed], J.block_var[i - n_freed] == 0,
-                              J.block_inside[i - n_freed] != 0, false, lane);
-    }
-}
-
-__global__ void __launch_bounds__(256, 2) occ_blocks_kernel(const OccLaunch* __restrict__ Lp)
-{
-    occ_blocks_stage(*Lp, blockIdx.x, gridDim.x);
-}
-
 // ---------------------------------------------------------------------- propagation --
 
-// propagate_block_to_coarsest_scale (multires_ofusion_core_impl.hpp:120-276), one warp per block
-__device__ void occ_up_best(OccD& parent, const OccD* ch, bool want_min)
-{
-    float best = want_min ? FLT_MAX : -FLT_MAX;
-    int bi = 0, nv = 0, no = 0;
-    for (int i = 0; i < 8; ++i) {
-        if (occ_valid(ch[i])) {
-            ++nv;
-            no += ch[i].observed ? 1 : 0;
-            const float fv = occ_field(ch[i]);
-            if (want_min ? (fv < best) : (fv > best)) {
-                best = fv;
-                bi = i;
-            }
-        }
-    }
-    if (nv > 0) {
-        parent = ch[bi];
-        parent.observed = (no == 8) ? 1 : 0;
-    }
-}
-
-__device__ void occ_up_mean(OccD& parent, const OccD* ch)
-{
-    float os = 0.0f, ws = 0.0f;
-    int n = 0;
-    for (int i = 0; i < 8; ++i)
-        if (occ_valid(ch[i])) {
-            ++n;
-            os += ch[i].occ;
-            ws += ch[i].weight;
-        }
-    if (n > 0) {
-        parent.occ = os / (float) n;
-        parent.weight = ceilf(ws / (float) n);
-        parent.observed = 0;
-    }
-}
-
-// Streaming forms of the two reductions: children in index order, the same comparisons and
-// sums as occ_up_best / occ_up_mean.
+// The reduction of 8 children to their parent's minimum (or maximum) data (multires_ofusion_core_impl.hpp:
+// 14-85): the first child with the least (greatest) field, observed if all 8 are; child 0 where no field
+// beats the bound. One thread adds the children in index order (up_best_add), or a group of 8 lanes holds
+// one each (occ_up_best8: the lane with the result returns true, with the data in d; none where no child is
+// valid).
 struct UpBest {
     float best;
     OccD pick;
@@ -1425,79 +1422,120 @@ __device__ __forceinline__ void up_best_add(UpBest& a, const OccD& c, bool want_
         }
     }
 }
+__device__ __forceinline__ bool occ_up_best8(const OccD& c, bool want_min, int lane, OccD& d)
+{
+    const unsigned group = 0xffu << (lane & 24);
+    const bool valid = occ_valid(c);
+    const unsigned nv = __ballot_sync(0xffffffffu, valid) & group;
+    const unsigned no = __ballot_sync(0xffffffffu, valid && c.observed) & group;
+    const float bound = want_min ? FLT_MAX : -FLT_MAX;
+    float best = valid ? occ_field(c) : bound;
+    const bool cand = want_min ? best < bound : best > bound; // a NaN is none
+    best = cand ? best : bound;
+    int at = cand ? (lane & 7) : 8;
+    for (int o = 1; o < 8; o <<= 1) {
+        const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oa = __shfl_xor_sync(0xffffffffu, at, o);
+        if ((want_min ? ob < best : ob > best) || (ob == best && oa < at)) {
+            best = ob;
+            at = oa;
+        }
+    }
+    d = c;
+    d.observed = no == group ? 1 : 0;
+    return nv != 0 && (lane & 7) == (at & 7); // none beat the bound: child 0
+}
 
+// propagate_block_to_coarsest_scale (multires_ofusion_core_impl.hpp:120-276), one warp per block. Scale 1 has
+// 64 parents, two for a lane, whose 8 children are loaded together; the coarser ones have 8 and 1, with a
+// lane for each child.
 __device__ void occ_propagate_block(const OccDevice& m, int b, int lane)
 {
     const OccBlockState st = m.block_state[b];
-    if (st.current_scale == kOccMaxScale)
-        return;
-    int cs = st.current_scale;
-    for (int ps = cs + 1; ps <= kOccMaxScale; ++ps) {
-        cs = ps - 1;
-        const int np = 8 >> ps;
+    for (int ps = st.current_scale + 1; ps <= kOccMaxScale; ++ps) {
+        const int cs = ps - 1;
+        const int lp = 3 - ps, np3 = 1 << (3 * lp); // 2^lp parents per axis
         OccD* pmin = blk_min(m, b, st.finest, ps);
         OccD* pmax = blk_max(m, b, st.finest, ps);
         OccD* pmean = blk_mean(m, b, ps);
         const OccD* cmean = blk_mean(m, b, cs);
-        const OccD* cmin = blk_min(m, b, st.finest, cs);
-        const OccD* cmax = blk_max(m, b, st.finest, cs);
         const bool first = ps == st.current_scale + 1;
         const bool do_mean = !(first && st.buffer_scale > st.current_scale);
-        for (int k = lane; k < np * np * np; k += 32) {
-            const int lp = 3 - ps; // np = 2^lp
-            const int x = k & (np - 1), y = (k >> lp) & (np - 1), z = k >> (2 * lp);
-            // ch[0] is visited first so that ties keep the lowest child index, as the array form
-            UpBest lo{FLT_MAX, OccD{0.0f, 0.0f, 0}, 0, 0}, hi{-FLT_MAX, OccD{0.0f, 0.0f, 0}, 0, 0};
-            float os = 0.0f, ws = 0.0f;
-            int nmean = 0;
-            bool lo_first = true, hi_first = true;
-            for (int c = 0; c < 8; ++c) {
+        if (ps == 1) { // the children are at the current scale: one set of data
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const int k = lane + 32 * r;
+                const int x = k & 3, y = (k >> 2) & 3, z = k >> 4;
+                OccD ch[8];
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                    ch[c] = cmean[(2 * x + (c & 1)) + ((2 * y + ((c >> 1) & 1)) << 3) + ((2 * z + (c >> 2)) << 6)];
+                UpBest lo{FLT_MAX, ch[0], 0, 0}, hi{-FLT_MAX, ch[0], 0, 0};
+                float os = 0.0f, ws = 0.0f;
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    if (occ_valid(ch[c])) {
+                        os += ch[c].occ;
+                        ws += ch[c].weight;
+                    }
+                    up_best_add(lo, ch[c], true);
+                    up_best_add(hi, ch[c], false);
+                }
+                if (lo.nv > 0) {
+                    if (do_mean)
+                        pmean[k] = OccD{os / (float) lo.nv, ceilf(ws / (float) lo.nv), 0};
+                    lo.pick.observed = hi.pick.observed = lo.no == 8 ? 1 : 0;
+                    pmin[k] = lo.pick;
+                    pmax[k] = hi.pick;
+                }
+            }
+        }
+        else {
+            const OccD* cmin = blk_min(m, b, st.finest, cs);
+            const OccD* cmax = blk_max(m, b, st.finest, cs);
+            for (int k0 = 0; k0 < np3; k0 += 4) {
+                const int k = k0 + (lane >> 3), c = lane & 7;
+                const bool on = k < np3;
+                const int x = k & ((1 << lp) - 1), y = (k >> lp) & ((1 << lp) - 1), z = k >> (2 * lp);
                 const int ci = (2 * x + (c & 1)) + ((2 * y + ((c >> 1) & 1)) << (lp + 1))
                     + ((2 * z + (c >> 2)) << (2 * (lp + 1)));
-                const OccD c0 = cmean[ci];
-                const OccD c1 = first ? c0 : cmin[ci];
-                const OccD c2 = first ? c0 : cmax[ci];
-                if (occ_valid(c0)) {
-                    ++nmean;
-                    os += c0.occ;
-                    ws += c0.weight;
+                OccD c0 = occ_default(), c1 = c0, c2 = c0;
+                if (on) {
+                    c0 = cmean[ci];
+                    c1 = first ? c0 : cmin[ci];
+                    c2 = first ? c0 : cmax[ci];
                 }
-                // the array form starts from index 0 when no child beats the initial bound
-                if (lo_first) {
-                    lo.pick = c1;
-                    lo_first = false;
+                const unsigned valid = __ballot_sync(0xffffffffu, occ_valid(c0)) >> (lane & 24);
+                float os = 0.0f, ws = 0.0f;
+                int nmean = 0;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) { // the sums in index order
+                    const float o = __shfl_sync(0xffffffffu, c0.occ, i, 8), w = __shfl_sync(0xffffffffu, c0.weight, i, 8);
+                    if ((valid >> i) & 1u) {
+                        ++nmean;
+                        os += o;
+                        ws += w;
+                    }
                 }
-                if (hi_first) {
-                    hi.pick = c2;
-                    hi_first = false;
-                }
-                up_best_add(lo, c1, true);
-                up_best_add(hi, c2, false);
-            }
-            if (do_mean && nmean > 0) {
-                OccD& p = pmean[k];
-                p.occ = os / (float) nmean;
-                p.weight = ceilf(ws / (float) nmean);
-                p.observed = 0;
-            }
-            if (lo.nv > 0) {
-                OccD r = lo.pick;
-                r.observed = (lo.no == 8) ? 1 : 0;
-                pmin[k] = r;
-            }
-            if (hi.nv > 0) {
-                OccD r = hi.pick;
-                r.observed = (hi.no == 8) ? 1 : 0;
-                pmax[k] = r;
+                if (on && c == 0 && do_mean && nmean > 0)
+                    pmean[k] = OccD{os / (float) nmean, ceilf(ws / (float) nmean), 0};
+                OccD d;
+                if (occ_up_best8(c1, true, lane, d) && on)
+                    pmin[k] = d;
+                if (occ_up_best8(c2, false, lane, d) && on)
+                    pmax[k] = d;
             }
         }
         __syncwarp();
     }
 }
 
-// Block propagation on the freed and the carver's blocks (one warp per block); the carver's
-// blocks also put their parents in the first propagation set (propagateToRoot's seeds).
-__device__ void occ_propagate_blocks_stage(const OccLaunch& L, int bid, int nbid)
+// freeBlock on the freed blocks and updateBlock on the carver's blocks (disjoint: the carver does not
+// descend below a free-space node), then the block's own propagation, one warp per block, all maps. A
+// block's propagation needs that block alone: in a stage of its own it read everything again (320x240: 42 +
+// 33 us as two launches, 57 as one; eight 1024x64 LiDAR maps: 102 + 64 and 127). The carver's blocks also put their parents in the first propagation
+// set (propagateToRoot's seeds).
+__device__ void occ_blocks_stage(const OccLaunch& L, int bid, int nbid)
 {
     __shared__ int pre[kOccMaxBatch + 1];
     const int total = batch_prefix(L, pre, [](const OccJob& J) {
@@ -1512,45 +1550,59 @@ __device__ void occ_propagate_blocks_stage(const OccLaunch& L, int bid, int nbid
         const OccDevice& m = J.m;
         const int n_freed = clamp_count(m.counters[kOccFreedN], m.block_capacity);
         const int i = idx - pre[j];
-        const int b = i < n_freed ? J.freed[i] : J.block_list[i - n_freed];
+        const bool free = i < n_freed;
+        const int b = free ? J.freed[i] : J.block_list[i - n_freed];
+        const bool low_var = free || J.block_var[i - n_freed] == 0;
+        const bool inside = free || J.block_inside[i - n_freed] != 0;
+        occ_process_block(L, J, b, low_var, inside, free, lane);
         occ_propagate_block(m, b, lane);
-        if (i >= n_freed && lane == 0)
+        if (!free && lane == 0)
             occ_set_insert(m, J.sets, m.block_state[b].parent, J.dyn->frame_id);
     }
 }
 
-__global__ void __launch_bounds__(256) occ_propagate_blocks_kernel(const OccLaunch* __restrict__ Lp)
+__global__ void __launch_bounds__(256, 3) occ_blocks_kernel(const OccLaunch* __restrict__ Lp)
 {
-    occ_propagate_blocks_stage(*Lp, blockIdx.x, gridDim.x);
+    grid_dep_wait();
+    occ_blocks_stage(*Lp, blockIdx.x, gridDim.x);
 }
 
-// updater::propagate_to_parent_node (multires_ofusion_core_impl.hpp:88-117)
-__device__ OccD occ_propagate_node(const OccDevice& m, int n, int timestamp)
+// updater::propagate_to_parent_node (multires_ofusion_core_impl.hpp:88-117) by a group of 8 lanes, a child
+// each (all 32 lanes call it; n < 0: an idle group). A child's data are three dependent loads, which one
+// thread for a node did eight times in turn. The node's maximum is returned to the group.
+__device__ OccD occ_propagate_node(const OccDevice& m, int n, int timestamp, int lane)
 {
-    m.node_ts[n] = timestamp;
-    OccD cmin[8], cmax[8];
-    for (int i = 0; i < 8; ++i) {
-        const int c = m.node_child[8 * (size_t) n + i];
-        if (c == -1) {
-            cmin[i] = occ_default();
-            cmax[i] = occ_default();
+    OccD cmin = occ_default(), cmax = occ_default(), mx = occ_default();
+    if (n >= 0) {
+        const int c = m.node_child[8 * (size_t) n + (lane & 7)];
+        mx = m.node_max[n];
+        if (c != -1) {
+            if (slot_is_block(c)) {
+                const int b = slot_block(c);
+                const int fin = m.block_state[b].finest;
+                cmin = blk_min(m, b, fin, kOccMaxScale)[0];
+                cmax = blk_max(m, b, fin, kOccMaxScale)[0];
+            }
+            else {
+                cmin = m.node_min[c];
+                cmax = m.node_max[c];
+            }
         }
-        else if (slot_is_block(c)) {
-            const int b = slot_block(c);
-            const int fin = m.block_state[b].finest;
-            cmin[i] = blk_min(m, b, fin, kOccMaxScale)[0];
-            cmax[i] = blk_max(m, b, fin, kOccMaxScale)[0];
-        }
-        else {
-            cmin[i] = m.node_min[c];
-            cmax[i] = m.node_max[c];
-        }
+        if ((lane & 7) == 0)
+            m.node_ts[n] = timestamp;
     }
-    OccD mn = m.node_min[n], mx = m.node_max[n];
-    occ_up_best(mn, cmin, true);
-    occ_up_best(mx, cmax, false);
-    m.node_min[n] = mn;
-    m.node_max[n] = mx;
+    OccD d;
+    if (occ_up_best8(cmin, true, lane, d) && n >= 0)
+        m.node_min[n] = d;
+    const bool mine = occ_up_best8(cmax, false, lane, d);
+    if (mine && n >= 0)
+        m.node_max[n] = d;
+    const unsigned who = (__ballot_sync(0xffffffffu, mine) >> (lane & 24)) & 0xffu;
+    const int src = (lane & 24) + (who ? __ffs(who) - 1 : 0);
+    const float occ = __shfl_sync(0xffffffffu, d.occ, src), weight = __shfl_sync(0xffffffffu, d.weight, src);
+    const int observed = __shfl_sync(0xffffffffu, d.observed, src);
+    if (who)
+        mx = OccD{occ, weight, observed};
     return mx;
 }
 
@@ -1577,44 +1629,71 @@ __device__ void occ_delete_children(const OccDevice& m, int n)
     }
 }
 
-// One depth of propagateToRoot over every map's propagation set at that depth.
-__device__ void occ_propagate_nodes_stage(const OccLaunch& L, int depth, int bid, int nbid)
+// Up to 4 nodes of a map's propagation set at one depth, first and on, by a warp: 8 lanes a node.
+__device__ __forceinline__ void occ_propagate_set(const OccJob& J, int depth, int first, int total, int lane)
 {
-    __shared__ int pre[kOccMaxBatch + 1];
-    const int total = batch_prefix(
-        L, pre, [depth](const OccJob& J) { return clamp_count(J.m.counters[kOccSetN + depth], J.m.node_capacity); });
-    for (int idx = bid * blockDim.x + threadIdx.x; idx < total; idx += nbid * blockDim.x) {
-        const int j = batch_find(pre, L.n, idx);
-        const OccJob& J = L.job[j];
-        const OccDevice& m = J.m;
-        const OccDyn& D = *J.dyn;
-        const int node = J.sets[(size_t) depth * m.node_capacity + (idx - pre[j])];
-        if (m.node_ts[node] == D.timestamp)
-            continue;
-        if (m.node_parent[node] < 0)
-            continue;
-        const OccD nd = occ_propagate_node(m, node, D.timestamp);
-        occ_set_insert(m, J.sets, m.node_parent[node], D.frame_id);
-        if (nd.observed && (double) occ_field(nd) <= 0.95 * -100.0) {
+    const OccDevice& m = J.m;
+    const OccDyn& D = *J.dyn;
+    const int idx = first + (lane >> 3);
+    int node = idx < total ? J.sets[(size_t) depth * m.node_capacity + idx] : -1;
+    int parent = -1;
+    if (node >= 0) {
+        parent = m.node_parent[node];
+        if (m.node_ts[node] == D.timestamp || parent < 0)
+            node = -1;
+    }
+    const OccD nd = occ_propagate_node(m, node, D.timestamp, lane);
+    if (node >= 0 && (lane & 7) == 0) {
+        occ_set_insert(m, J.sets, parent, D.frame_id);
+        if (nd.observed && occ_field(nd) <= kOccFreeField) {
             occ_delete_children(m, node);
             atomicAdd(&m.counters[kOccPruned], 1);
         }
+    }
+    __syncwarp();
+}
+
+// One depth of propagateToRoot over every map's propagation set at that depth.
+__device__ void occ_propagate_nodes_stage(const OccLaunch& L, int depth, int bid, int nbid)
+{
+    __shared__ int pre[kOccMaxBatch + 1]; // in warps' shares of 4 nodes
+    const int total = batch_prefix(L, pre, [depth](const OccJob& J) {
+        return (clamp_count(J.m.counters[kOccSetN + depth], J.m.node_capacity) + 3) / 4;
+    });
+    const int n_warps = (nbid * blockDim.x) >> 5;
+    for (int idx = (bid * blockDim.x + threadIdx.x) >> 5; idx < total; idx += n_warps) {
+        const int j = batch_find(pre, L.n, idx);
+        const OccJob& J = L.job[j];
+        occ_propagate_set(J, depth, 4 * (idx - pre[j]), clamp_count(J.m.counters[kOccSetN + depth], J.m.node_capacity),
+                          threadIdx.x & 31);
     }
 }
 
 __global__ void occ_propagate_nodes_kernel(const OccLaunch* __restrict__ Lp, int depth)
 {
+    grid_dep_wait();
     occ_propagate_nodes_stage(*Lp, depth, blockIdx.x, gridDim.x);
 }
 
-__global__ void occ_propagate_root_kernel(const OccLaunch* __restrict__ Lp)
+// The last depths of propagateToRoot, from depth up to the root, a cluster of CTAs for each map with its
+// barrier between the depths. A depth d holds at most 8^d nodes, so the upper ones are a few warps' work
+// whose launch and first loads cost more than the nodes (10 to 12 us each as launches of the whole GPU, 5 to
+// 6 here).
+__global__ void __launch_bounds__(kOccClusterThreads) occ_propagate_top_kernel(const OccLaunch* __restrict__ Lp, int depth)
 {
+    grid_dep_wait();
     const OccLaunch& L = *Lp;
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= L.n)
-        return;
-    const OccJob& J = L.job[j];
-    occ_propagate_node(J.m, 0, J.dyn->timestamp);
+    const OccJob& J = L.job[blockIdx.x / kOccCluster];
+    const int lane = threadIdx.x & 31;
+    const int warp = (blockIdx.x % kOccCluster) * (kOccClusterThreads / 32) + (threadIdx.x >> 5);
+    for (int d = depth; d > 0; --d) {
+        const int total = clamp_count(J.m.counters[kOccSetN + d], J.m.node_capacity);
+        for (int first = 4 * warp; first < total; first += 4 * kOccCluster * (kOccClusterThreads / 32))
+            occ_propagate_set(J, d, first, total, lane);
+        occ_cluster_sync();
+    }
+    if (warp == 0)
+        occ_propagate_node(J.m, lane < 8 ? 0 : -1, J.dyn->timestamp, lane);
 }
 
 // ------------------------------------------------------------- one persistent launch --
@@ -1709,19 +1788,16 @@ __global__ void __launch_bounds__(256, 2) occ_persistent_kernel(const OccLaunch*
         occ_blocks_stage(L, bid, nbid);
         ok = occ_grid_sync(bar, phase);
     }
-    if (ok) {
-        occ_propagate_blocks_stage(L, bid, nbid);
-        ok = occ_grid_sync(bar, phase);
-    }
     for (int d = L.max_block_depth - 1; ok && d > 0; --d) {
         occ_propagate_nodes_stage(L, d, bid, nbid);
         ok = occ_grid_sync(bar, phase);
     }
-    if (bid == 0 && threadIdx.x < L.n) {
-        const OccJob& J = L.job[threadIdx.x];
+    if (bid == 0) {
+        const int j = threadIdx.x >> 3;
+        const OccJob& J = L.job[min(j, L.n - 1)];
         if (ok)
-            occ_propagate_node(J.m, 0, J.dyn->timestamp);
-        else
+            occ_propagate_node(J.m, j < L.n ? 0 : -1, J.dyn->timestamp, lane);
+        else if (j < L.n && (threadIdx.x & 7) == 0)
             atomicOr(&J.m.counters[kOccError], kOccErrTimeout);
     }
 }
@@ -1852,6 +1928,21 @@ void occ_scratch_free(se_gpu_occ_map* om)
     s = OccScratch();
 }
 
+// The least float chord whose ratio to the voxel diagonal, (float) (chord / (sqrt(3) res)) with the
+// division in double, is at least ratio. The ratio grows with the chord, so chord >= bound is the same test.
+static float lidar_scale_bound(float res, float ratio)
+{
+    const auto reaches = [res, ratio](float chord) {
+        return (float) ((double) chord / (std::sqrt(3.0) * (double) res)) >= ratio;
+    };
+    float c = (float) ((double) ratio * std::sqrt(3.0) * (double) res);
+    while (c > 0.0f && reaches(std::nextafterf(c, 0.0f)))
+        c = std::nextafterf(c, 0.0f);
+    while (c < INFINITY && !reaches(c))
+        c = std::nextafterf(c, INFINITY);
+    return c;
+}
+
 static OccJob occ_job(const se_gpu_occ_map* om)
 {
     const OccScratch& s = om->scratch;
@@ -1878,6 +1969,8 @@ static OccJob occ_job(const se_gpu_occ_map* om)
     J.tau_max = m.cfg.tau_max_factor * m.res;
     J.sigma_min = m.cfg.sigma_min_factor * m.res;
     J.sigma_max = m.cfg.sigma_max_factor * m.res;
+    for (int i = 0; i < 3; ++i)
+        J.lidar_bounds[i] = lidar_scale_bound(m.res, 1.5f * (float) (1 << i));
     return J;
 }
 
@@ -1932,33 +2025,33 @@ static se_gpu_status occ_enqueue(const OccLaunch& L, const OccLaunch* Ld, const 
     const int n = L.n;
     const int carve = sms * t.ctas[kTileCarve], list = sms * t.ctas[kTileList], blocks = sms * t.ctas[kTileBlocks];
     if (step_dev)
-        occ_begin_dev_kernel<<<n, 64, 0, stream>>>(Ld, step_dev);
+        launch_chained(occ_begin_dev_kernel, n, 64, stream, Ld, step_dev);
     else
-        occ_begin_kernel<<<n, 64, 0, stream>>>(Ld, step);
-    occ_pixels_kernel<<<dim3((npx + 255) / 256, n), 256, 0, stream>>>(Ld);
+        launch_chained(occ_begin_kernel, n, 64, stream, Ld, step);
+    launch_chained(occ_pixels_kernel, dim3((npx + 255) / 256, n), 256, stream, Ld);
     for (int l = 1; l < L.sensor.levels; ++l)
-        occ_pool_level_kernel<<<dim3((npx + 255) / 256, 2 * n), 256, 0, stream>>>(Ld, l);
-    occ_root_kernel<<<n, 32, 0, stream>>>(Ld);
-    for (int d = 1; d <= L.max_block_depth; ++d) {
+        launch_chained(occ_pool_level_kernel, dim3((npx + 255) / 256, 2 * n), 256, stream, Ld, l);
+    const int head = L.max_block_depth < kOccTopCarve ? L.max_block_depth : kOccTopCarve;
+    SE_CUDA_TRY(launch_clusters(occ_carve_top_kernel, n, stream, Ld, head));
+    for (int d = head + 1; d <= L.max_block_depth; ++d) {
         OCC_MARK(kTileCarve);
-        occ_carve_kernel<<<carve, 128, 0, stream>>>(Ld, d);
+        launch_chained(occ_carve_kernel, carve, 128, stream, Ld, d);
     }
     OCC_MARK(kTileList);
-    occ_nodes_kernel<<<list, 256, 0, stream>>>(Ld);
+    launch_chained(occ_nodes_kernel, list, 256, stream, Ld);
     for (int it = 0; it <= L.max_block_depth; ++it) {
         OCC_MARK(kTileList);
-        occ_free_nodes_kernel<<<list, 256, 0, stream>>>(Ld, it);
+        launch_chained(occ_free_nodes_kernel, list, 256, stream, Ld, it);
     }
     OCC_MARK(kTileBlocks);
-    occ_blocks_kernel<<<blocks, 256, 0, stream>>>(Ld);
-    OCC_MARK(kTileBlocks);
-    occ_propagate_blocks_kernel<<<blocks, 256, 0, stream>>>(Ld);
-    for (int d = L.max_block_depth - 1; d > 0; --d) {
+    launch_chained(occ_blocks_kernel, blocks, 256, stream, Ld);
+    int top = L.max_block_depth - 1;
+    for (; top > kOccTopPropagate; --top) {
         OCC_MARK(kTileList);
-        occ_propagate_nodes_kernel<<<list, 256, 0, stream>>>(Ld, d);
+        launch_chained(occ_propagate_nodes_kernel, list, 256, stream, Ld, top);
     }
     OCC_MARK(-1);
-    occ_propagate_root_kernel<<<1, 32, 0, stream>>>(Ld);
+    SE_CUDA_TRY(launch_clusters(occ_propagate_top_kernel, n, stream, Ld, top));
     SE_CUDA_TRY(cudaGetLastError());
     return SE_GPU_OK;
 }

@@ -177,6 +177,7 @@ struct OccJob {
     int* sets;          // per depth, node_capacity entries each
     OccDyn* dyn;
     float tau_min, tau_max, sigma_min, sigma_max;
+    float lidar_bounds[3]; // see lidar_integration_scale
 };
 
 // Everything a launch needs except the per-frame inputs, passed by value (__grid_constant__).
