@@ -382,6 +382,9 @@ SE_GPU_API se_gpu_status se_gpu_map_field_interp(const se_gpu_map* map, int64_t 
                                       float* values_dev, int* valid_dev, void* stream);
 SE_GPU_API se_gpu_status se_gpu_map_field_grad(const se_gpu_map* map, int64_t n, const float* points_W_dev,
                                     float* grads_dev, int* valid_dev, void* stream);
+/* The same (grad 0: n values, otherwise n gradients) with one byte a point, 1 or 0, for the validity. */
+SE_GPU_API se_gpu_status se_gpu_map_field_query(const se_gpu_map* map, int64_t n, const float* points_W_dev, int grad,
+                                     float* out_dev, uint8_t* valid_dev, void* stream);
 /* Allocated-block AABB in voxels (Octree::aabb(), inclusive). Synchronous; returns
  * SE_GPU_OK with *empty = 1 when no block is allocated. */
 SE_GPU_API se_gpu_status se_gpu_map_aabb(const se_gpu_map* map, int32_t mn[3], int32_t mx[3], int* empty);

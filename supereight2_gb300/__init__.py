@@ -139,6 +139,7 @@ SIGNATURES = {
                                                C.POINTER(C.c_int64)]),
     "se_gpu_map_field_interp": (C.c_int, [_VP, C.c_int64, _VP, _VP, _VP, _VP]),
     "se_gpu_map_field_grad": (C.c_int, [_VP, C.c_int64, _VP, _VP, _VP, _VP]),
+    "se_gpu_map_field_query": (C.c_int, [_VP, C.c_int64, _VP, C.c_int, _VP, _VP, _VP]),
     "se_gpu_map_aabb": (C.c_int, [_VP, C.POINTER(C.c_int32), C.POINTER(C.c_int32),
                                   C.POINTER(C.c_int)]),
     "se_gpu_render_depth": (C.c_int, [_VP, C.POINTER(_Pinhole), _F16, _VP, _VP]),
@@ -207,7 +208,8 @@ def _stream(stream):
     if stream is not None:
         return C.c_void_p(int(stream))
     import torch
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # (the same as torch.cuda.current_stream().cuda_stream without a Stream object)
+    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def _dptr(t, dtype, shape=None, name="tensor"):
@@ -216,7 +218,7 @@ def _dptr(t, dtype, shape=None, name="tensor"):
         raise SeGpuError(f"{name} must be a CUDA tensor")
     if t.dtype != dtype or not t.is_contiguous():
         raise SeGpuError(f"{name} must be a contiguous {dtype} tensor")
-    if shape is not None and tuple(t.shape) != tuple(shape):
+    if shape is not None and t.shape != tuple(shape):
         raise SeGpuError(f"{name} has shape {tuple(t.shape)}, expected {tuple(shape)}")
     return C.c_void_p(t.data_ptr())
 
@@ -492,12 +494,12 @@ class Map:
         import torch
         n = points_W.shape[0]
         p = _dptr(points_W, torch.float32, (n, 3), "points_W")
-        out = torch.zeros((n, 3) if grad else (n,), dtype=torch.float32, device=points_W.device)
-        valid = torch.zeros(n, dtype=torch.int32, device=points_W.device)
-        fn = self._L.se_gpu_map_field_grad if grad else self._L.se_gpu_map_field_interp
-        _check(fn(self.h, n, p, C.c_void_p(out.data_ptr()), C.c_void_p(valid.data_ptr()),
-                  _stream(stream)), "field query")
-        return out, valid.bool()
+        # the kernel writes every element of both
+        out = torch.empty((n, 3) if grad else (n,), dtype=torch.float32, device=points_W.device)
+        valid = torch.empty(n, dtype=torch.bool, device=points_W.device)
+        _check(self._L.se_gpu_map_field_query(self.h, n, p, grad, out.data_ptr(), valid.data_ptr(),
+                                              _stream(stream)), "field query")
+        return out, valid
 
     def aabb(self):
         mn = (C.c_int32 * 3)()

@@ -123,7 +123,8 @@ __global__ void __launch_bounds__(128, 6) raycast_normal_kernel(MapDevice m, Pin
 // the raycast.
 template <int S, bool MR, bool GRAD>
 __global__ void __launch_bounds__(128) field_query_kernel(MapDevice m, int n, const float* __restrict__ pts,
-                                                          float* __restrict__ out, int* __restrict__ valid)
+                                                          float* __restrict__ out, int* __restrict__ valid,
+                                                          uint8_t* __restrict__ valid8)
 {
     __shared__ int sh_bt[GRAD ? 8 * 128 : 1];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -150,6 +151,8 @@ __global__ void __launch_bounds__(128) field_query_kernel(MapDevice m, int n, co
             ok = field_interp<S>(m, p, v);
         out[i] = ok ? v : 0.0f;
     }
+    if (valid8)
+        valid8[i] = ok ? 1 : 0;
     if (valid)
         valid[i] = ok ? 1 : 0;
 }
@@ -228,7 +231,7 @@ extern "C" se_gpu_status se_gpu_raycast(const se_gpu_map* map, const se_gpu_pinh
 }
 
 static se_gpu_status field_query(const se_gpu_map* map, int64_t n, const float* pts, float* out, int* valid,
-                                 void* stream_p, int grad)
+                                 uint8_t* valid8, void* stream_p, int grad)
 {
     if (!map || n < 0 || n > (1ll << 31) - 1 || (n > 0 && (!pts || !out))) {
         set_last_error("se_gpu_map_field_%s: invalid argument", grad ? "grad" : "interp");
@@ -246,9 +249,9 @@ static se_gpu_status field_query(const se_gpu_map* map, int64_t n, const float* 
 #define SE_QUERY_LAUNCH(S_, MR_)                                                                                     \
     do {                                                                                                            \
         if (grad)                                                                                                   \
-            field_query_kernel<S_, MR_, true><<<blocks, 128, 0, stream>>>(map->dev, (int) n, pts, out, valid);       \
+            field_query_kernel<S_, MR_, true><<<blocks, 128, 0, stream>>>(map->dev, (int) n, pts, out, valid, valid8); \
         else                                                                                                        \
-            field_query_kernel<S_, MR_, false><<<blocks, 128, 0, stream>>>(map->dev, (int) n, pts, out, valid);      \
+            field_query_kernel<S_, MR_, false><<<blocks, 128, 0, stream>>>(map->dev, (int) n, pts, out, valid, valid8); \
     } while (0)
     if (map->dev.storage == SE_GPU_STORAGE_F32 && !mr)
         SE_QUERY_LAUNCH(SE_GPU_STORAGE_F32, false);
@@ -266,11 +269,17 @@ static se_gpu_status field_query(const se_gpu_map* map, int64_t n, const float* 
 extern "C" se_gpu_status se_gpu_map_field_interp(const se_gpu_map* map, int64_t n, const float* pts, float* values,
                                                  int* valid, void* stream)
 {
-    return field_query(map, n, pts, values, valid, stream, 0);
+    return field_query(map, n, pts, values, valid, nullptr, stream, 0);
 }
 
 extern "C" se_gpu_status se_gpu_map_field_grad(const se_gpu_map* map, int64_t n, const float* pts, float* grads,
                                                int* valid, void* stream)
 {
-    return field_query(map, n, pts, grads, valid, stream, 1);
+    return field_query(map, n, pts, grads, valid, nullptr, stream, 1);
+}
+
+extern "C" se_gpu_status se_gpu_map_field_query(const se_gpu_map* map, int64_t n, const float* pts, int grad, float* out,
+                                                uint8_t* valid, void* stream)
+{
+    return field_query(map, n, pts, out, nullptr, valid, stream, grad != 0);
 }

@@ -274,7 +274,7 @@ __device__ bool field_interp(const MapDevice& m, F3 p_W, float& out)
 // [base - 1, base + 2]^3 (at most 2 per axis) are looked up once into bt (this thread's 8
 // entries, bt[k * bs] for k = x | y << 1 | z << 2 block offsets), then the 32 voxel loads are
 // independent of one another; a failed sample fails the query. (One after another, 50,000 queries
-// took 42 us with their interpolations, now 12.)
+// took 42 us with their interpolations, now 14.)
 template <int S>
 __device__ bool field_grad_batched(const MapDevice& m, BlockCache& c, F3 p_W, F3& g, int* bt, int bs)
 {
