@@ -37,6 +37,7 @@ constexpr int kOccPathLevels = 10;  // levels 4..13: nodes of 16^3 to 8192^3 vox
 // Every answer is the root descent's.
 struct OccCursor {
     int* path;
+    uint64_t* near; // a whole warp's leaves, see occ_seek_warp
     int px, py, pz; // the voxel of the path (masked to the map)
     int low;        // path entries of levels low..log2_size are valid
     int slot;       // occ_leaf's answer inside the box (bx, by, bz) / mask
@@ -47,9 +48,10 @@ struct OccCursor {
 
 __device__ __forceinline__ int& occ_path(const OccCursor& c, int level) { return c.path[(level - 4) * kOccCtaThreads]; }
 
-__device__ __forceinline__ void occ_cursor_init(OccCursor& c, const OccDevice& m, int* path)
+__device__ __forceinline__ void occ_cursor_init(OccCursor& c, const OccDevice& m, int* path, uint64_t* near)
 {
     c.path = path;
+    c.near = near;
     c.px = c.py = c.pz = 0;
     c.low = m.log2_size;
     occ_path(c, m.log2_size) = 0;
@@ -226,6 +228,18 @@ __device__ __forceinline__ unsigned occ_votes(bool b) { return (__ballot_sync(kO
 // The value that lane k of this lane's group holds.
 __device__ __forceinline__ float occ_from(float v, int k) { return __shfl_sync(kOccWarp, v, (threadIdx.x & 24) | (k & 7)); }
 
+// The same over the kLanes lanes that sample a ray, a group or the whole warp.
+template <int kLanes>
+__device__ __forceinline__ unsigned occ_sample_votes(bool b)
+{
+    return kLanes == 32 ? __ballot_sync(kOccWarp, b) : occ_votes(b);
+}
+template <int kLanes>
+__device__ __forceinline__ float occ_sample_from(float v, int k)
+{
+    return kLanes == 32 ? __shfl_sync(kOccWarp, v, k & 31) : occ_from(v, k);
+}
+
 // The data of a voxel at `scale` (BlockMultiRes::data or a leaf node's): false where nothing is
 // allocated or the block's current scale is coarser.
 __device__ __forceinline__ bool occ_data_at(const OccDevice& m, OccCursor& c, int x, int y, int z, int scale, OccD& d)
@@ -240,15 +254,135 @@ __device__ __forceinline__ bool occ_data_at(const OccDevice& m, OccCursor& c, in
     return true;
 }
 
+// ---- lookups of a warp that has one ray
+//
+// Each lane has a sample of its own, so lanes' lookups differ in length; left to themselves the lanes part
+// and the rest of the turn runs lane by lane. Here the warp stays together: every lane calls, those with
+// `run` set look up. The leaves found last are kept for the warp, one for each of the block coordinates'
+// low two bits on each axis (a turn's samples and their cells span at most four blocks an axis); a descent
+// is one to four dependent loads. An entry is one 64-bit word (lanes store and load it whole): the block
+// coordinates (10 bits an axis), the slot (28 bits and whether it is a block), and a block's scales or a
+// node's level. A slot beyond its field is not kept.
+constexpr int kOccNear = 64;
+constexpr uint64_t kOccNearEmpty = ~0ull; // no entry: a slot is less
+
+// The leaf at a voxel (masked to the map) for the lanes with `need` set, from level L of the path down: its
+// slot, and level | current scale << 4 | finest << 8 | (the path's new lowest level, 0: not walked) << 12. A
+// function of its own, for the code's size: the rays that it serves are few and wait for instructions.
+static __device__ __noinline__ int2 occ_find_warp(const OccDevice& m, uint64_t* near, int* path, int xm, int ym, int zm, int L,
+                                                  bool need)
+{
+    const uint32_t tag = (uint32_t) (xm >> 3) | ((uint32_t) (ym >> 3) << 10) | ((uint32_t) (zm >> 3) << 20);
+    volatile uint64_t* entry = near + (((xm >> 3) & 3) | (((ym >> 3) & 3) << 2) | (((zm >> 3) & 3) << 4));
+    int slot = -1, level = 3, scales = 0, low = 0;
+    bool go = need;
+    if (need) {
+        const uint64_t e = *entry;
+        if ((uint32_t) (e >> 34) == tag && e != kOccNearEmpty) {
+            go = false;
+            slot = (int) ((e >> 5) & 0xfffffffu);
+            if (e & 1u) {
+                slot = -2 - slot;
+                scales = (int) (e >> 1) & 15; // current | finest << 2
+            }
+            else {
+                level = (int) (e >> 1) & 15;
+            }
+        }
+    }
+    if (__any_sync(kOccWarp, go)) {
+        const bool walk = go;
+        int n = walk ? path[(L - 4) * kOccCtaThreads] : 0;
+        while (__any_sync(kOccWarp, go)) {
+            if (go) {
+                const int s = L - 1;
+                const int ch =
+                    m.node_child[8 * (size_t) n + (((xm >> s) & 1) | (((ym >> s) & 1) << 1) | (((zm >> s) & 1) << 2))];
+                if (ch == -1) {
+                    const bool leaf = occ_no_children(m, n);
+                    slot = leaf ? n : -1;
+                    level = leaf ? L : s;
+                    go = false;
+                }
+                else if (slot_is_block(ch)) {
+                    slot = ch;
+                    level = s;
+                    go = false;
+                }
+                else {
+                    n = ch;
+                    L = s;
+                    path[(L - 4) * kOccCtaThreads] = n;
+                }
+            }
+        }
+        if (walk)
+            low = L;
+        if (walk && slot != -1) {
+            uint64_t e = (uint64_t) (level << 1);
+            int idx = slot;
+            if (slot_is_block(slot)) {
+                idx = slot_block(slot);
+                const OccBlockState& st = m.block_state[idx];
+                scales = st.current_scale | st.finest << 2;
+                e = (uint64_t) (scales << 1 | 1);
+            }
+            if (idx < 0xfffffff)
+                *entry = e | ((uint64_t) tag << 34) | ((uint64_t) idx << 5);
+        }
+    }
+    __syncwarp();
+    return make_int2(slot, level | (scales & 3) << 4 | (scales >> 2) << 8 | low << 12);
+}
+
+__device__ __forceinline__ int occ_seek_warp(const OccDevice& m, OccCursor& c, int x, int y, int z, bool run)
+{
+    const int mk = m.size - 1;
+    const int xm = x & mk, ym = y & mk, zm = z & mk;
+    const bool miss = run && (((xm ^ c.bx) | (ym ^ c.by) | (zm ^ c.bz)) & c.mask) != 0;
+    if (!__any_sync(kOccWarp, miss))
+        return c.slot;
+    const int2 f = occ_find_warp(m, c.near, c.path, xm, ym, zm,
+                                 max(c.low, 32 - __clz((xm ^ c.px) | (ym ^ c.py) | (zm ^ c.pz))), miss);
+    if (miss) {
+        const int slot = f.x;
+        if (f.y >> 12) {
+            c.px = xm;
+            c.py = ym;
+            c.pz = zm;
+            c.low = f.y >> 12;
+        }
+        if (slot_is_block(slot)) {
+            c.cur = (f.y >> 4) & 3;
+            c.fin = (f.y >> 8) & 3;
+        }
+        c.slot = slot;
+        c.mask = ~((1 << (f.y & 15)) - 1);
+        c.bx = xm & c.mask;
+        c.by = ym & c.mask;
+        c.bz = zm & c.mask;
+        c.nd = occ_default();
+        if (slot >= 0)
+            c.nd = node_data(m, slot);
+    }
+    __syncwarp();
+    return c.slot;
+}
+
 // visitor::getInterp multi-res with get_neighbours on an occupancy octree (leaf nodes take part), desired
 // scale 0, lane k of a group taking corner k; called by the whole warp, for the groups with `run` set.
 // aabb: the map's seven box words, in shared memory. The sums pair up as the serial expression's, so
 // every lane of the group gets its value.
+template <bool kWarp>
 __device__ __forceinline__ bool occ_interp(const OccDevice& m, OccCursor& c, const int* aabb, F3 vf, bool run, float& out,
                                            int& returned_scale)
 {
     const int k = threadIdx.x & 7;
-    const int q = run ? occ_seek(m, c, (int) vf.x, (int) vf.y, (int) vf.z) : -1;
+    int q = -1;
+    if constexpr (kWarp)
+        q = occ_seek_warp(m, c, (int) vf.x, (int) vf.y, (int) vf.z, run);
+    else if (run)
+        q = occ_seek(m, c, (int) vf.x, (int) vf.y, (int) vf.z);
     const bool q_block = slot_is_block(q);
     int scale = q_block ? c.cur : 0;
     run = run && q != -1;
@@ -267,9 +401,12 @@ __device__ __forceinline__ bool occ_interp(const OccDevice& m, OccCursor& c, con
                 fail = true;
             else if (b0 + stride >= m.size || b1 + stride >= m.size || b2 + stride >= m.size || b0 < 0 || b1 < 0 || b2 < 0)
                 skip = true;
-            else
-                have = occ_data_at(m, c, b0 + ((k & 1) ? stride : 0), b1 + ((k & 2) ? stride : 0), b2 + ((k & 4) ? stride : 0),
-                                   scale, e);
+            else {
+                const int x = b0 + ((k & 1) ? stride : 0), y = b1 + ((k & 2) ? stride : 0), z = b2 + ((k & 4) ? stride : 0);
+                if constexpr (kWarp) // run is the warp's: one ray
+                    occ_seek_warp(m, c, x, y, z, true);
+                have = occ_data_at(m, c, x, y, z, scale, e);
+            }
         }
         const bool all_have = occ_votes(have) == 0xffu, all_valid = occ_votes(occ_valid(e)) == 0xffu;
         // ((f0 tcx + f1 tx) tcy + (f2 tcx + f3 tx) ty) tcz + (...) tz
@@ -297,39 +434,6 @@ __device__ __forceinline__ bool occ_interp(const OccDevice& m, OccCursor& c, con
         }
     }
     return ok;
-}
-
-// Whether occ_interp has a value at vf, by one lane alone.
-__device__ __forceinline__ bool occ_interp_exists(const OccDevice& m, OccCursor& c, const int* aabb, F3 vf)
-{
-    const int q = occ_seek(m, c, (int) vf.x, (int) vf.y, (int) vf.z);
-    if (q == -1)
-        return false;
-    bool valid = false;
-#pragma unroll 1
-    for (int scale = slot_is_block(q) ? c.cur : 0; scale <= kOccMaxScale; ++scale) {
-        const int stride = 1 << scale;
-        const float inv = occ_inv_size(scale);
-        const int b0 = stride * (int) (inv * vf.x - 0.5f), b1 = stride * (int) (inv * vf.y - 0.5f),
-                  b2 = stride * (int) (inv * vf.z - 0.5f);
-        if (aabb[6] || b0 < aabb[0] || b1 < aabb[1] || b2 < aabb[2] || b0 > aabb[3] || b1 > aabb[4] || b2 > aabb[5])
-            break;
-        if (b0 + stride >= m.size || b1 + stride >= m.size || b2 + stride >= m.size || b0 < 0 || b1 < 0 || b2 < 0)
-            continue;
-        bool have = true;
-        valid = true;
-#pragma unroll 1
-        for (int k = 0; k < 8 && have; ++k) {
-            OccD e = occ_default();
-            have = occ_data_at(m, c, b0 + ((k & 1) ? stride : 0), b1 + ((k & 2) ? stride : 0), b2 + ((k & 4) ? stride : 0), scale,
-                               e);
-            valid = valid && occ_valid(e);
-        }
-        if (have)
-            break;
-        valid = false;
-    }
-    return valid;
 }
 
 // The 32 gradient samples in the reference's order: per axis a selector of {base - stride, base,
@@ -443,6 +547,69 @@ __device__ __forceinline__ int occ_box_steps(const OccCursor& c, F3 v, F3 dv, fl
     const float lim = fminf(fminf((rx - 0.25f) / fabsf(dv.x), (ry - 0.25f) / fabsf(dv.y)), (rz - 0.25f) / fabsf(dv.z));
     const float n = fminf(lim / step, (float) kOccSkipMax) - 1.0f;
     return n > 0.0f ? (int) n : 0; // also 0 for a NaN
+}
+
+// Whether occ_interp has a value at vf, each lane with `run` set for its own point. The blocks of a cell's
+// corners (one, or two along an axis the cell crosses a block's face on) are looked up into `tab` (the
+// lane's 8 words of shared memory, kOccCtaThreads apart): a block and whether its initial data holds at the
+// scale, or -1 / -2 for a leaf node with / without valid data. The corners' weights then load together.
+__device__ __forceinline__ bool occ_interp_exists(const OccDevice& m, OccCursor& c, const int* aabb, F3 vf, bool run, int* tab)
+{
+    const int q = occ_seek_warp(m, c, (int) vf.x, (int) vf.y, (int) vf.z, run);
+    run = run && q != -1;
+    int scale = slot_is_block(q) ? c.cur : 0;
+    bool ok = false;
+    while (__any_sync(kOccWarp, run)) {
+        const int stride = 1 << scale;
+        int b0 = 0, b1 = 0, b2 = 0;
+        bool have = false;
+        if (run) {
+            const float inv = occ_inv_size(scale);
+            b0 = stride * (int) (inv * vf.x - 0.5f);
+            b1 = stride * (int) (inv * vf.y - 0.5f);
+            b2 = stride * (int) (inv * vf.z - 0.5f);
+            if (aabb[6] || b0 < aabb[0] || b1 < aabb[1] || b2 < aabb[2] || b0 > aabb[3] || b1 > aabb[4] || b2 > aabb[5])
+                run = false;
+            else
+                have = !(b0 + stride >= m.size || b1 + stride >= m.size || b2 + stride >= m.size || b0 < 0 || b1 < 0 || b2 < 0);
+        }
+        const int two = ((b0 & 7) + stride > 7 ? 1 : 0) | ((b1 & 7) + stride > 7 ? 2 : 0) | ((b2 & 7) + stride > 7 ? 4 : 0);
+#pragma unroll 1
+        for (int k = 0; k < 8; ++k) {
+            const bool look = have && (k & ~two) == 0;
+            if (!__any_sync(kOccWarp, look))
+                continue;
+            const int slot = occ_seek_warp(m, c, b0 + ((k & 1) ? stride : 0), b1 + ((k & 2) ? stride : 0),
+                                           b2 + ((k & 4) ? stride : 0), look);
+            if (look) {
+                have = slot != -1 && !(slot_is_block(slot) && c.cur > scale);
+                tab[k * kOccCtaThreads] = slot_is_block(slot) ? (slot_block(slot) << 1) | (scale < c.fin ? 1 : 0)
+                                                              : (occ_valid(c.nd) ? -1 : -2);
+            }
+        }
+        bool valid = true;
+        if (have) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int e = tab[(k & two) * kOccCtaThreads];
+                float w = e == -1 ? 1.0f : 0.0f;
+                if (e >= 0) {
+                    const OccD* d = (e & 1) ? &m.block_state[e >> 1].init_data
+                                            : blk_mean(m, e >> 1, scale)
+                            + blk_voxel_idx(b0 + ((k & 1) ? stride : 0), b1 + ((k & 2) ? stride : 0), b2 + ((k & 4) ? stride : 0),
+                                            scale);
+                    w = d->weight;
+                }
+                valid = valid && w != 0.0f;
+            }
+        }
+        if (run) {
+            ok = have && valid;
+            run = !have && ++scale <= kOccMaxScale;
+        }
+        __syncwarp();
+    }
+    return ok;
 }
 
 // compute_map_intersection (raycaster_impl.hpp:85-173)
@@ -591,16 +758,36 @@ __device__ __forceinline__ void occ_advance_ray(const OccDevice& m, OccCursor& c
 // a field above -0.2, the end of the ray) is taken up, the ones before it only move the ray on, the ones
 // after it are dropped. Where a search falls in a leaf octant without data (an unallocated octant, an
 // unobserved node) the samples that are certain to stay in it are passed without a lookup.
+//
+// Along the edge of what has been seen a ray meets hundreds of points whose interpolation has no value (up
+// to 269 in a view of the room). After kOccTries of them in a row it is put aside (`susp`, with the state
+// that the search needs), and RESUME takes it up: a ray has a warp, a turn 32 samples, and each lane looks
+// for itself whether its sample has a value.
+struct OccSuspended {
+    float t, t_far, value_tt, t_ptt;
+    int bits; // why | has_tt << 2 | (scale_tt + 1) << 3
+};
+constexpr int kOccTries = 2;
+template <bool RESUME>
 __device__ __forceinline__ bool occ_raycast(const OccDevice& m, OccCursor& c, const OccRes& r, const int* aabb, F3 o, F3 d,
-                                            float t_far, bool active, F3& hit, int& scale_out)
+                                            float t_far, bool active, int* tab, OccSuspended& susp, bool& suspended, F3& hit,
+                                            int& scale_out)
 {
-    const int lane = threadIdx.x & 7;
+    constexpr int kLanes = RESUME ? 32 : 8; // the samples of a turn
+    const int lane = threadIdx.x & (kLanes - 1);
     bool valid = active;
     float t = 0.0f;
-    if (active)
-        t = occ_map_intersection(m, o, d, t_far, valid);
-    const int max_scale = min(7, m.log2_size - 1);
-    occ_advance_ray(m, c, r, o, d, t, t_far, max_scale, valid);
+    suspended = false;
+    if constexpr (RESUME) {
+        t = susp.t;
+        t_far = susp.t_far;
+    }
+    else {
+        if (active)
+            t = occ_map_intersection(m, o, d, t_far, valid);
+        const int max_scale = min(7, m.log2_size - 1);
+        occ_advance_ray(m, c, r, o, d, t, t_far, max_scale, valid);
+    }
     const float step = m.res / 2;
     const F3 dv = mul(rot(m.T_MW, d), r.inv); // voxels per unit of t, for the box skips only
     float value_t = 0.0f, value_tt = 0.0f;
@@ -614,16 +801,20 @@ __device__ __forceinline__ bool occ_raycast(const OccDevice& m, OccCursor& c, co
     hit = f3(0.0f, 0.0f, 0.0f);
     bool want = false; // the sample at t waits for its interpolation
     float value = 0.0f;
-    // interpolations that the search made in a row without a value: along the edge of what has been seen a
-    // ray meets hundreds of such points (up to 269 in a view of the room), so after kOccTries each lane
-    // looks for itself whether its sample has one
-    constexpr int kOccTries = 2;
-    int failed = 0;
+    int failed = 0; // interpolations that the search made in a row without a value
+    if constexpr (RESUME) {
+        why = susp.bits & 3;
+        has_tt = (susp.bits >> 2) & 1;
+        scale_tt = (susp.bits >> 3) - 1;
+        value_tt = susp.value_tt;
+        t_ptt = susp.t_ptt;
+        failed = kOccTries;
+    }
     for (;;) {
         const bool take = mode != kDone && !want, find = mode == kFind;
         float tk = t; // sample `lane`, its steps accumulated one by one
 #pragma unroll
-        for (int j = 0; j < 7; ++j)
+        for (int j = 0; j < kLanes - 1; ++j)
             if (j < lane)
                 tk += step;
         // the samples that the loops would reach: the first is not tested again
@@ -631,25 +822,32 @@ __device__ __forceinline__ bool occ_raycast(const OccDevice& m, OccCursor& c, co
         bool has = false;
         int pass = 0; // samples certain to lie in the same octant without data
         float fk = 0.0f;
-        if (take && there) {
-            const F3 p_M = occ_to_map(m, r, add(o, mul(tk, d)));
-            // the march's Map::getData has no bounds check (Safe::Off)
-            if (!find || occ_in_map(m, p_M)) {
-                const F3 vk = occ_sample_voxel(r, p_M);
-                const OccD data = occ_get_data_voxel(m, c, (int) vk.x, (int) vk.y, (int) vk.z);
-                has = occ_valid(data);
-                fk = occ_field(data);
-                if (find && !has && lane == 7 && !slot_is_block(c.slot))
-                    pass = occ_box_steps(c, vk, dv, step);
-                if (find && has && failed >= kOccTries)
-                    has = occ_interp_exists(m, c, aabb, vk);
+        const F3 p_M = occ_to_map(m, r, add(o, mul(tk, d)));
+        // the march's Map::getData has no bounds check (Safe::Off)
+        const bool look = take && there && (!find || occ_in_map(m, p_M));
+        const F3 vk = occ_sample_voxel(r, p_M);
+        if constexpr (RESUME)
+            occ_seek_warp(m, c, (int) vk.x, (int) vk.y, (int) vk.z, look);
+        if (look) {
+            const OccD data = occ_get_data_voxel(m, c, (int) vk.x, (int) vk.y, (int) vk.z);
+            has = occ_valid(data);
+            fk = occ_field(data);
+            if (find && !has && lane == kLanes - 1 && !slot_is_block(c.slot))
+                pass = occ_box_steps(c, vk, dv, step);
+        }
+        if constexpr (RESUME) {
+            const bool probe = find && has && failed >= kOccTries;
+            if (__any_sync(kOccWarp, probe)) {
+                const bool exists = occ_interp_exists(m, c, aabb, vk, probe, tab);
+                if (probe)
+                    has = exists;
             }
         }
-        const unsigned events = occ_votes(take && there && (find ? has : !has || fk > -0.2f));
-        const unsigned gone = occ_votes(!there), data_bits = occ_votes(has);
-        const int e = events ? __ffs(events) - 1 : 7; // the sample to act on, or the last one
-        const float t_e = occ_from(tk, e), f_e = occ_from(fk, e), t_b = occ_from(tk, e - 1), f_b = occ_from(fk, e - 1);
-        pass = __shfl_sync(kOccWarp, pass, threadIdx.x | 7);
+        const unsigned events = occ_sample_votes<kLanes>(take && there && (find ? has : !has || fk > -0.2f));
+        const unsigned gone = occ_sample_votes<kLanes>(!there), data_bits = occ_sample_votes<kLanes>(has);
+        const int e = events ? __ffs(events) - 1 : kLanes - 1; // the sample to act on, or the last one
+        const float t_e = occ_sample_from<kLanes>(tk, e), f_e = occ_sample_from<kLanes>(fk, e), t_b = occ_sample_from<kLanes>(tk, e - 1), f_b = occ_sample_from<kLanes>(fk, e - 1);
+        pass = __shfl_sync(kOccWarp, pass, threadIdx.x | (kLanes - 1));
         if (take) {
             if (events) {
                 t = t_e;
@@ -710,12 +908,13 @@ __device__ __forceinline__ bool occ_raycast(const OccDevice& m, OccCursor& c, co
             continue;
         int sc = scale_tt;
         const F3 v = occ_sample_voxel(r, occ_to_map(m, r, add(o, mul(t, d))));
-        const bool ok = occ_interp(m, c, aabb, v, want, value, sc);
+        const bool ok = occ_interp<RESUME>(m, c, aabb, v, want, value, sc);
         if (!want)
             continue;
         want = false;
         if (mode == kFind) {
-            failed = ok ? 0 : failed + 1;
+            if (!RESUME) // a ray once put aside looks ahead from then on
+                failed = ok ? 0 : failed + 1;
             if (ok) {
                 t_pt = t;
                 value_t = value;
@@ -731,6 +930,10 @@ __device__ __forceinline__ bool occ_raycast(const OccDevice& m, OccCursor& c, co
                     mode = kDone;
                     has_tt = false;
                     found = why == kWhyNoData;
+                }
+                else if (!RESUME && failed >= kOccTries) {
+                    suspended = true;
+                    mode = kDone;
                 }
             }
         }
@@ -757,6 +960,10 @@ __device__ __forceinline__ bool occ_raycast(const OccDevice& m, OccCursor& c, co
             }
         }
     }
+    if (suspended) {
+        susp = OccSuspended{t, t_far, value_tt, t_ptt, why | (has_tt ? 4 : 0) | ((scale_tt + 1) << 3)};
+        return false;
+    }
     if (found) {
         scale_out = 0;
         return true;
@@ -771,42 +978,77 @@ __device__ __forceinline__ bool occ_raycast(const OccDevice& m, OccCursor& c, co
     return false;
 }
 
-// raycaster::raycast_volume for occupancy maps: normals are -normalize(grad F)
-__global__ void __launch_bounds__(kOccCtaThreads) occ_raycast_kernel(OccDevice m, OccRes r, Pinhole s, Tf T_WS,
-                                                                     float* __restrict__ pts, float* __restrict__ nrm,
-                                                                     int8_t* __restrict__ scale)
+// raycaster::raycast_volume for occupancy maps, in three launches: the rays, four to a warp; the rays put
+// aside (RESUME), a warp for a ray; the normals. In between a pixel's outputs hold its ray's state, marked in
+// the normal's x by a value that is none (kOccHitMark: a hit without its normal; kOccSuspendedMark).
+//
+// Why: rays along the edge of what has been seen take 50 to 120 turns of the loop, the others 7, and lie
+// together. Four to a warp, 1 % of the warps were most of the time, with the rest of the GPU idle, and all
+// of them waited for instructions (65 KB of code as one kernel; 42, 50 and 19 as three). A view of a room,
+// 2 cm, with its integration: 320x240 820 us as one kernel, 744 with the rays put aside, 704 with the normals
+// apart too; a 160x120 view after eight LiDAR scans 577, 590 and 567.
+constexpr float kOccSuspendedMark = 2.0f, kOccHitMark = 3.0f;
+template <bool RESUME>
+__global__ void __launch_bounds__(kOccCtaThreads) occ_raycast_kernel(const __grid_constant__ OccDevice m, OccRes r, Pinhole s,
+                                                                     Tf T_WS, float* __restrict__ pts,
+                                                                     float* __restrict__ nrm, int8_t* __restrict__ scale)
 {
+    grid_dep_wait();
     __shared__ int sh_path[kOccPathLevels * kOccCtaThreads];
-    __shared__ float sh_grad[kOccCtaThreads / 8][33];
+    __shared__ int sh_tab[RESUME ? 8 * kOccCtaThreads : 1];
+    __shared__ uint64_t sh_near[RESUME ? kOccNear * (kOccCtaThreads / 32) : 1];
     __shared__ int sh_aabb[7];
     if (threadIdx.x < 7)
         sh_aabb[threadIdx.x] = m.aabb[threadIdx.x];
     __syncthreads();
     const int warp = threadIdx.x >> 5, ray = (threadIdx.x >> 3) & 3, lane = threadIdx.x & 7;
-    const int x = blockIdx.x * 4 + (warp & 1) * 2 + (ray & 1);
-    const int y = blockIdx.y * 4 + (warp >> 1) * 2 + (ray >> 1);
+    int x, y;
+    if constexpr (RESUME) {
+        const int i = blockIdx.x * (kOccCtaThreads / 32) + warp;
+        if (i >= s.w * s.h || nrm[3 * (size_t) i] != kOccSuspendedMark)
+            return;
+        x = i % s.w;
+        y = i / s.w;
+    }
+    else {
+        x = blockIdx.x * 4 + (warp & 1) * 2 + (ray & 1);
+        y = blockIdx.y * 4 + (warp >> 1) * 2 + (ray >> 1);
+    }
     const bool in_image = x < s.w && y < s.h; // rays past the edge stay for the warp's votes
     OccCursor c;
-    occ_cursor_init(c, m, sh_path + threadIdx.x);
+    occ_cursor_init(c, m, sh_path + threadIdx.x, RESUME ? sh_near + kOccNear * warp : nullptr);
+    if constexpr (RESUME) {
+        for (int k = threadIdx.x & 31; k < kOccNear; k += 32)
+            c.near[k] = kOccNearEmpty;
+        __syncwarp();
+    }
     const size_t idx = (size_t) x + (size_t) y * s.w;
     const F3 ray_S = back_project(s, (float) x, (float) y);
     const F3 nS = normalized(ray_S);
     const F3 dir_W = rot(T_WS, nS);
     const F3 origin = f3(T_WS.t[0], T_WS.t[1], T_WS.t[2]);
-    F3 hit, g, p = f3(0.0f, 0.0f, 0.0f), n = f3(0.0f, 0.0f, 0.0f);
+    F3 hit, p = f3(0.0f, 0.0f, 0.0f), n = f3(0.0f, 0.0f, 0.0f);
     int sc = 0;
-    const bool is_hit = occ_raycast(m, c, r, sh_aabb, origin, dir_W, s.far_plane / nS.z, in_image, hit, sc);
-    const bool has_grad = occ_grad(m, c, occ_to_voxel_f(m, r, hit), is_hit, sh_grad[threadIdx.x >> 3], g);
-    if (is_hit)
+    OccSuspended susp;
+    bool suspended;
+    if constexpr (RESUME)
+        susp = OccSuspended{pts[3 * idx], pts[3 * idx + 1], pts[3 * idx + 2], nrm[3 * idx + 1],
+                            __float_as_int(nrm[3 * idx + 2])};
+    const bool is_hit = occ_raycast<RESUME>(m, c, r, sh_aabb, origin, dir_W, s.far_plane / nS.z, in_image,
+                                            RESUME ? sh_tab + threadIdx.x : nullptr, susp, suspended, hit, sc);
+    if (is_hit) {
         p = hit;
-    else
-        sc = 0;
-    if (has_grad) {
-        g = f3(g.x / m.res, g.y / m.res, g.z / m.res);
-        const float nn = sqrtf(dot(g, g));
-        n = nn > 0.0f ? f3(-(g.x / nn), -(g.y / nn), -(g.z / nn)) : f3(-g.x, -g.y, -g.z);
+        n.x = kOccHitMark;
     }
-    if (!in_image)
+    else {
+        sc = 0;
+    }
+    if (suspended) {
+        p = f3(susp.t, susp.t_far, susp.value_tt);
+        n = f3(kOccSuspendedMark, susp.t_ptt, __int_as_float(susp.bits));
+    }
+    __syncwarp(); // every lane has read the ray's state
+    if (!in_image || (RESUME && ray != 0))
         return;
     if (lane < 3)
         pts[3 * idx + lane] = lane == 0 ? p.x : lane == 1 ? p.y : p.z;
@@ -814,6 +1056,34 @@ __global__ void __launch_bounds__(kOccCtaThreads) occ_raycast_kernel(OccDevice m
         nrm[3 * idx + lane - 3] = lane == 3 ? n.x : lane == 4 ? n.y : n.z;
     else if (lane == 6 && scale)
         scale[idx] = (int8_t) sc;
+}
+
+// The normals at the hits, which occ_raycast_kernel has marked.
+__global__ void __launch_bounds__(kOccCtaThreads) occ_normal_kernel(const __grid_constant__ OccDevice m, OccRes r, int w, int h,
+                                                                    const float* __restrict__ pts, float* __restrict__ nrm)
+{
+    grid_dep_wait();
+    __shared__ int sh_path[kOccPathLevels * kOccCtaThreads];
+    __shared__ float sh_grad[kOccCtaThreads / 8][33];
+    const int warp = threadIdx.x >> 5, ray = (threadIdx.x >> 3) & 3, lane = threadIdx.x & 7;
+    const int x = blockIdx.x * 4 + (warp & 1) * 2 + (ray & 1);
+    const int y = blockIdx.y * 4 + (warp >> 1) * 2 + (ray >> 1);
+    const size_t idx = (size_t) x + (size_t) y * w;
+    const bool is_hit = x < w && y < h && nrm[3 * idx] == kOccHitMark;
+    if (!__any_sync(kOccWarp, is_hit))
+        return;
+    OccCursor c;
+    occ_cursor_init(c, m, sh_path + threadIdx.x, nullptr);
+    F3 hit = f3(0.0f, 0.0f, 0.0f), g, n = f3(0.0f, 0.0f, 0.0f);
+    if (is_hit)
+        hit = f3(pts[3 * idx], pts[3 * idx + 1], pts[3 * idx + 2]);
+    if (occ_grad(m, c, occ_to_voxel_f(m, r, hit), is_hit, sh_grad[threadIdx.x >> 3], g)) {
+        g = f3(g.x / m.res, g.y / m.res, g.z / m.res);
+        const float nn = sqrtf(dot(g, g));
+        n = nn > 0.0f ? f3(-(g.x / nn), -(g.y / nn), -(g.z / nn)) : f3(-g.x, -g.y, -g.z);
+    }
+    if (is_hit && lane < 3)
+        nrm[3 * idx + lane] = lane == 0 ? n.x : lane == 1 ? n.y : n.z;
 }
 
 se_gpu_status occ_raycast_volume(const se_gpu_occ_map* om, const se_gpu_pinhole& sensor, const float* T_WS16,
@@ -826,7 +1096,11 @@ se_gpu_status occ_raycast_volume(const se_gpu_occ_map* om, const se_gpu_pinhole&
         if (om->dev.T_MW.R[i] != ((i % 4 == 0) ? 1.0f : 0.0f))
             r.translation = 0;
     ProfScope ps(kProfRaycast, stream);
-    occ_raycast_kernel<<<grid, kOccCtaThreads, 0, stream>>>(om->dev, r, s, tf_from16(T_WS16), pts, nrm, scale);
+    launch_chained(occ_raycast_kernel<false>, grid, kOccCtaThreads, stream, om->dev, r, s, tf_from16(T_WS16), pts, nrm, scale);
+    constexpr int kWarps = kOccCtaThreads / 32;
+    launch_chained(occ_raycast_kernel<true>, (s.w * s.h + kWarps - 1) / kWarps, kOccCtaThreads, stream, om->dev, r, s,
+                   tf_from16(T_WS16), pts, nrm, scale);
+    launch_chained(occ_normal_kernel, grid, kOccCtaThreads, stream, om->dev, r, s.w, s.h, pts, nrm);
     SE_CUDA_TRY(cudaGetLastError());
     return SE_GPU_OK;
 }
