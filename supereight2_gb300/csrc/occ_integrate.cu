@@ -153,6 +153,20 @@ static_assert(0.95 * -100.0 == (double) kOccFreeField);
 
 // ------------------------------------------------------------------ per-pixel inputs --
 
+// A pooled depth pixel in 8 bytes: the minimum and maximum (both positive, or NaN), with what is known of
+// the window (0 all, 1 some, 2 none of its pixels) in their signs. Of the sigma image only the maximum is
+// asked for. (With 16 bytes each, a crossing flag that no query reads among them, the pyramids of eight
+// 1024x64 scans took 51 us and the carver 175 after them; so 30 and 143.)
+__device__ __forceinline__ float2 pool_pack(float mn, float mx, int known)
+{
+    return make_float2(__uint_as_float(__float_as_uint(mn) | (known == 2 ? 0x80000000u : 0u)),
+                       __uint_as_float(__float_as_uint(mx) | (known == 1 ? 0x80000000u : 0u)));
+}
+__device__ __forceinline__ int pool_known(float2 p)
+{
+    return __float_as_int(p.x) < 0 ? 2 : (__float_as_int(p.y) < 0 ? 1 : 0);
+}
+
 // uncert::depth_sigma with the linear model, and level 0 of both pooling images
 // (Pixel::knownPixel / unknownPixel: min = FLT_MAX, max = FLT_MIN, the smallest normal float)
 __device__ __forceinline__ void occ_pixel(const OccLaunch& L, int j, int i)
@@ -168,8 +182,8 @@ __device__ __forceinline__ void occ_pixel(const OccLaunch& L, int j, int i)
         sg = v < J.sigma_min ? J.sigma_min : (J.sigma_max < v ? J.sigma_max : v); // std::clamp
     }
     J.sigma[i] = sg;
-    J.pool_depth[i] = d <= 0.0f ? make_float4(FLT_MAX, FLT_MIN, 0.0f, 2.0f) : make_float4(d, d, 0.0f, 0.0f);
-    J.pool_sigma[i] = sg <= 0.0f ? make_float4(FLT_MAX, FLT_MIN, 0.0f, 2.0f) : make_float4(sg, sg, 0.0f, 0.0f);
+    J.pool_depth[i] = d <= 0.0f ? pool_pack(FLT_MAX, FLT_MIN, 2) : pool_pack(fabsf(d), fabsf(d), 0); // a NaN's sign goes
+    J.pool_sigma[i] = sg <= 0.0f ? FLT_MIN : sg;
 }
 
 __global__ void occ_pixels_kernel(const OccLaunch* __restrict__ Lp)
@@ -187,41 +201,35 @@ __global__ void occ_pixels_kernel(const OccLaunch* __restrict__ Lp)
 // Level 1 (3x3 windows, dense_pooling_image_impl.hpp:92-165 / 423-478) or level l >= 2 (the four
 // overlapping windows of level l - 1, :167-213 / 480-565) of both images of every map; the LiDAR
 // image wraps around in u.
-__device__ __forceinline__ void occ_pool_pixel(const OccLaunch& L, int level, int j, int which, int i)
+__device__ __forceinline__ void occ_pool_pixel(const OccLaunch& L, int level, int j, int i)
 {
     const int w = L.sensor.w, h = L.sensor.h, npx = w * h;
     const bool wrap = L.sensor.lidar != 0;
     const OccJob& J = L.job[j];
-    float4* base = which ? J.pool_sigma : J.pool_depth;
-    const float4* P = base + (size_t) (level - 1) * npx;
+    const float2* P = J.pool_depth + (size_t) (level - 1) * npx;
+    const float* S = J.pool_sigma + (size_t) (level - 1) * npx;
     const int x = i % w, y = i / w;
-    float4 p = make_float4(FLT_MAX, FLT_MIN, 1.0f, 0.0f); // crossingKnownPixel
+    // (from FLT_MIN, as the queries start: a window of NaN pixels alone has no maximum)
+    float mn = FLT_MAX, mx = FLT_MIN, sg = FLT_MIN;
+    int uf = 0, all;
     if (level == 1) {
-        if (y >= 1 && y < h - 1 && (wrap || (x >= 1 && x < w - 1)))
-            p.z = 0.0f;
         const int top = y > 0 ? y - 1 : 0, bottom = y < h - 1 ? y + 1 : h - 1;
         const int left = x > 0 ? x - 1 : (wrap ? w - 1 : 0);
         const int right = x < w - 1 ? x + 1 : (wrap ? 0 : w - 1);
         const int xs[9] = {x, left, x, right, right, right, x, left, left};
         const int ys[9] = {y, top, top, top, y, bottom, bottom, bottom, y};
-        float mn = FLT_MAX, mx = -FLT_MAX;
-        int uf = 0;
+        all = 18;
+#pragma unroll
         for (int k = 0; k < 9; ++k) {
-            const float4 q = P[xs[k] + ys[k] * w];
-            mn = fminf(mn, q.x);
-            mx = fmaxf(mx, q.y);
-            uf += (int) q.w;
+            const float2 q = P[xs[k] + ys[k] * w];
+            mn = fminf(mn, fabsf(q.x));
+            mx = fmaxf(mx, fabsf(q.y));
+            uf += pool_known(q);
+            sg = fmaxf(sg, S[xs[k] + ys[k] * w]);
         }
-        p.x = mn;
-        p.y = mx;
-        if (uf == 18)
-            p.w = 2.0f;
-        else if (uf > 0)
-            p.w = 1.0f;
     }
     else {
-        const int s = 1 << (level - 1);
-        const int s_half = s / 2;
+        const int s_half = 1 << (level - 2);
         int left, right, top, bottom;
         if (x - s_half < 0)
             left = wrap ? w + (x - s_half) : 0;
@@ -239,20 +247,19 @@ __device__ __forceinline__ void occ_pool_pixel(const OccLaunch& L, int level, in
             bottom = h - 1;
         else
             bottom = y + s_half;
-        const float4 a = P[left + top * w], b = P[right + top * w], c = P[left + bottom * w],
-                     d = P[right + bottom * w];
-        p.x = fminf(fminf(a.x, b.x), fminf(c.x, d.x));
-        p.y = fmaxf(fmaxf(a.y, b.y), fmaxf(c.y, d.y));
-        const int uf = (int) a.w + (int) b.w + (int) c.w + (int) d.w;
-        if (uf == 8)
-            p.w = 2.0f;
-        else if (uf > 0)
-            p.w = 1.0f;
-        // the window crossing the border stays crossing; windows inside are inside
-        if (y >= s && y < h - s && x >= s && x < w - s)
-            p.z = 0.0f;
+        const int at[4] = {left + top * w, right + top * w, left + bottom * w, right + bottom * w};
+        all = 8;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float2 q = P[at[k]];
+            mn = fminf(mn, fabsf(q.x));
+            mx = fmaxf(mx, fabsf(q.y));
+            uf += pool_known(q);
+            sg = fmaxf(sg, S[at[k]]);
+        }
     }
-    base[(size_t) level * npx + i] = p;
+    J.pool_depth[(size_t) level * npx + i] = pool_pack(mn, mx, uf == all ? 2 : (uf > 0 ? 1 : 0));
+    J.pool_sigma[(size_t) level * npx + i] = sg;
 }
 
 __global__ void occ_pool_level_kernel(const OccLaunch* __restrict__ Lp, int level)
@@ -261,10 +268,10 @@ __global__ void occ_pool_level_kernel(const OccLaunch* __restrict__ Lp, int leve
     const OccLaunch& L = *Lp;
     const int npx = L.sensor.w * L.sensor.h;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y >> 1;
+    const int j = blockIdx.y;
     if (i >= npx || j >= L.n)
         return;
-    occ_pool_pixel(L, level, j, blockIdx.y & 1, i);
+    occ_pool_pixel(L, level, j, i);
 }
 
 struct PoolQuery {
@@ -307,7 +314,7 @@ __device__ __forceinline__ int pool_index(int k, int nu, int u_min, int u_max, i
     return uf + w * v;
 }
 
-__device__ PoolPair pool_bounding_box(const float4* __restrict__ pool_d, const float4* __restrict__ pool_s, int w,
+__device__ PoolPair pool_bounding_box(const float2* __restrict__ pool_d, const float* __restrict__ pool_s, int w,
                                       int h, int max_level, bool wrap, int u_min, int u_max, int v_min, int v_max,
                                       int lane)
 {
@@ -322,16 +329,18 @@ __device__ PoolPair pool_bounding_box(const float4* __restrict__ pool_d, const f
     const bool u_wrap = wrap && (u_min < 0 || u_max > w - 1);
     const int nu = visit_count(u_min, u_max, s, step), nv = visit_count(v_min, v_max, s, step);
     const int n = nu * nv;
-    const float4* Ld = pool_d + (size_t) level * w * h;
-    const float* Ls = reinterpret_cast<const float*>(pool_s + (size_t) level * w * h) + 1; // .y = max
+    const float2* Ld = pool_d + (size_t) level * w * h;
+    const float* Ls = pool_s + (size_t) level * w * h;
     float mn = FLT_MAX, mx = FLT_MIN, smx = FLT_MIN; // Pixel::knownPixel
     bool all_unknown = true, any_part = false;
     for (int k = lane; k < n; k += 64) {
         const int i0 = pool_index(k, nu, u_min, u_max, v_min, v_max, s, step, w, u_wrap);
         const bool two = k + 32 < n;
         const int i1 = two ? pool_index(k + 32, nu, u_min, u_max, v_min, v_max, s, step, w, u_wrap) : i0;
-        const float4 p0 = Ld[i0], p1 = Ld[i1];
-        const float s0 = Ls[4 * (size_t) i0], s1 = Ls[4 * (size_t) i1];
+        const float2 q0 = Ld[i0], q1 = Ld[i1];
+        const float s0 = Ls[i0], s1 = Ls[i1];
+        const int known0 = pool_known(q0), known1 = pool_known(q1);
+        const float2 p0 = make_float2(fabsf(q0.x), fabsf(q0.y)), p1 = make_float2(fabsf(q1.x), fabsf(q1.y));
         if (mx < p0.y)
             mx = p0.y;
         if (mn > p0.x)
@@ -344,8 +353,8 @@ __device__ PoolPair pool_bounding_box(const float4* __restrict__ pool_d, const f
             smx = s0;
         if (smx < s1)
             smx = s1;
-        all_unknown = all_unknown && p0.w == 2.0f && p1.w == 2.0f;
-        any_part = any_part || p0.w >= 1.0f || p1.w >= 1.0f;
+        all_unknown = all_unknown && known0 == 2 && known1 == 2;
+        any_part = any_part || known0 != 0 || known1 != 0;
     }
     for (int o = 16; o > 0; o >>= 1) {
         const float omn = __shfl_xor_sync(0xffffffffu, mn, o), omx = __shfl_xor_sync(0xffffffffu, mx, o);
@@ -369,7 +378,7 @@ __device__ PoolPair pool_bounding_box(const float4* __restrict__ pool_d, const f
 
 // conservativeQuery (dense_pooling_image_impl.hpp:295-347; Ouster: 734-781 clips only v) of the
 // depth and the sigma pyramids, by a whole warp with uniform arguments
-__device__ PoolPair conservative_query(const float4* __restrict__ pool_d, const float4* __restrict__ pool_s, int w,
+__device__ PoolPair conservative_query(const float2* __restrict__ pool_d, const float* __restrict__ pool_s, int w,
                                        int h, int max_level, bool wrap, int u_min, int v_min, int u_max, int v_max,
                                        int lane)
 {
@@ -553,14 +562,14 @@ __device__ void occ_root(const OccLaunch& L, int j, int lane)
     const OccJob& J = L.job[j];
     const int w = L.sensor.w, h = L.sensor.h;
     const int max_level = L.sensor.levels - 1;
-    const float4* Lmax = J.pool_depth + (size_t) max_level * w * h;
+    const float2* Lmax = J.pool_depth + (size_t) max_level * w * h;
     const int s = 1 << (max_level - 1);
     // rows s, 3s, ... and the last row h - s - 1; the same for the columns
     const int nv = visit_count(0, h - 1, s, 2 * s), nu = visit_count(0, w - 1, s, 2 * s);
     float mv = 0.0f;
     for (int k = lane; k < nu * nv; k += 32) {
         const int u = min(s + (k % nu) * 2 * s, w - s - 1), v = min(s + (k / nu) * 2 * s, h - s - 1);
-        const float m = Lmax[u + w * v].y;
+        const float m = fabsf(Lmax[u + w * v].y);
         if (mv < m)
             mv = m;
     }
@@ -1761,10 +1770,8 @@ __global__ void __launch_bounds__(256, 2) occ_persistent_kernel(const OccLaunch*
         ok = occ_grid_sync(bar, phase);
     }
     for (int l = 1; ok && l < L.sensor.levels; ++l) {
-        for (long long k = tid; k < 2 * L.n * npx; k += nthreads) {
-            const int jj = (int) (k / npx);
-            occ_pool_pixel(L, l, jj >> 1, jj & 1, (int) (k % npx));
-        }
+        for (long long k = tid; k < L.n * npx; k += nthreads)
+            occ_pool_pixel(L, l, (int) (k / npx), (int) (k % npx));
         ok = occ_grid_sync(bar, phase);
     }
     if (ok) {
@@ -1893,12 +1900,13 @@ static se_gpu_status occ_scratch_reserve(se_gpu_occ_map* om, int w, int h)
     cudaFree(s.pool_depth);
     cudaFree(s.pool_sigma);
     s.sigma = nullptr;
-    s.pool_depth = s.pool_sigma = nullptr;
+    s.pool_depth = nullptr;
+    s.pool_sigma = nullptr;
     const int levels = pooling_levels(w, h);
     const size_t npx = (size_t) w * h;
     SE_CUDA_TRY(cudaMalloc(&s.sigma, npx * sizeof(float)));
-    SE_CUDA_TRY(cudaMalloc(&s.pool_depth, (size_t) levels * npx * sizeof(float4)));
-    SE_CUDA_TRY(cudaMalloc(&s.pool_sigma, (size_t) levels * npx * sizeof(float4)));
+    SE_CUDA_TRY(cudaMalloc(&s.pool_depth, (size_t) levels * npx * sizeof(float2)));
+    SE_CUDA_TRY(cudaMalloc(&s.pool_sigma, (size_t) levels * npx * sizeof(float)));
     s.w = w;
     s.h = h;
     s.levels = levels;
@@ -2030,7 +2038,7 @@ static se_gpu_status occ_enqueue(const OccLaunch& L, const OccLaunch* Ld, const 
         launch_chained(occ_begin_kernel, n, 64, stream, Ld, step);
     launch_chained(occ_pixels_kernel, dim3((npx + 255) / 256, n), 256, stream, Ld);
     for (int l = 1; l < L.sensor.levels; ++l)
-        launch_chained(occ_pool_level_kernel, dim3((npx + 255) / 256, 2 * n), 256, stream, Ld, l);
+        launch_chained(occ_pool_level_kernel, dim3((npx + 255) / 256, n), 256, stream, Ld, l);
     const int head = L.max_block_depth < kOccTopCarve ? L.max_block_depth : kOccTopCarve;
     SE_CUDA_TRY(launch_clusters(occ_carve_top_kernel, n, stream, Ld, head));
     for (int d = head + 1; d <= L.max_block_depth; ++d) {

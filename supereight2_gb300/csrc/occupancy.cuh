@@ -164,8 +164,8 @@ struct OccDyn {
 struct OccJob {
     OccDevice m;
     float* sigma;
-    float4* pool_depth; // levels * w * h of (min, max, crossing, known)
-    float4* pool_sigma;
+    float2* pool_depth; // levels * w * h, see pool_pack
+    float* pool_sigma;  // levels * w * h maxima
     float* max_value;   // [0] max pooled depth, [1] max_depth_value
     int* frontier[2];
     int* block_list;    // slot block index
@@ -200,8 +200,8 @@ struct OccStep {
 struct OccScratch {
     int w = 0, h = 0, levels = 0;
     float* sigma = nullptr;
-    float4* pool_depth = nullptr;
-    float4* pool_sigma = nullptr;
+    float2* pool_depth = nullptr;
+    float* pool_sigma = nullptr;
     float* max_value = nullptr;
     int* frontier[2] = {nullptr, nullptr};
     int* block_list = nullptr;
