@@ -846,7 +846,9 @@ def _lidar_bench(se, torch, dev, K, warmup, flush):
     scans = LIDAR_MAPS * K
     bd = 5  # 256^3 voxels: blocks at depth 5
     levels = 6  # pooling levels of a 64-row image
-    launches = 1 + 1 + (levels - 1) + 1 + bd + 1 + (bd + 1) + 2 + (bd - 1) + 1
+    # begin, pixels, pooling levels, the carver's first two depths, its others, node list, free levels,
+    # blocks, the propagation's depths past 4, the others with the root
+    launches = 1 + 1 + (levels - 1) + 1 + max(bd - 2, 0) + 1 + (bd + 1) + 1 + max(bd - 5, 0) + 1
     return {
         "workload": f"{LIDAR_MAPS} multi-res occupancy maps (256^3 voxels at {LIDAR_RES} m, 8^3 blocks), "
                     f"LiDAR {spec.height}x{spec.width} (+-22.5 deg, {spec.near_plane}-{spec.far_plane} m), "
