@@ -552,7 +552,8 @@ __device__ __forceinline__ int occ_box_steps(const OccCursor& c, F3 v, F3 dv, fl
 // Whether occ_interp has a value at vf, each lane with `run` set for its own point. The blocks of a cell's
 // corners (one, or two along an axis the cell crosses a block's face on) are looked up into `tab` (the
 // lane's 8 words of shared memory, kOccCtaThreads apart): a block and whether its initial data holds at the
-// scale, or -1 / -2 for a leaf node with / without valid data. The corners' weights then load together.
+// scale, or -1 / -2 for a leaf node with / without valid data: from the warp's leaves where all eight are
+// there, otherwise one after another. The corners' weights then load together.
 __device__ __forceinline__ bool occ_interp_exists(const OccDevice& m, OccCursor& c, const int* aabb, F3 vf, bool run, int* tab)
 {
     const int q = occ_seek_warp(m, c, (int) vf.x, (int) vf.y, (int) vf.z, run);
@@ -574,17 +575,38 @@ __device__ __forceinline__ bool occ_interp_exists(const OccDevice& m, OccCursor&
                 have = !(b0 + stride >= m.size || b1 + stride >= m.size || b2 + stride >= m.size || b0 < 0 || b1 < 0 || b2 < 0);
         }
         const int two = ((b0 & 7) + stride > 7 ? 1 : 0) | ((b1 & 7) + stride > 7 ? 2 : 0) | ((b2 & 7) + stride > 7 ? 4 : 0);
+        // the warp's leaves first, the corners' entries read together
+        bool known = have;
+        if (have) {
+            const uint32_t x0 = b0 >> 3, x1 = (b0 + stride) >> 3, y0 = b1 >> 3, y1 = (b1 + stride) >> 3, z0 = b2 >> 3,
+                           z1 = (b2 + stride) >> 3;
+            bool fine = true;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const uint32_t x = (k & 1) ? x1 : x0, y = (k & 2) ? y1 : y0, z = (k & 4) ? z1 : z0;
+                const uint64_t e = *(volatile uint64_t*) (c.near + ((x & 3) | ((y & 3) << 2) | ((z & 3) << 4)));
+                const uint32_t low = (uint32_t) e;
+                known = known && (uint32_t) (e >> 34) == (x | (y << 10) | (z << 20)) && (low & 1u) && e != kOccNearEmpty;
+                fine = fine && (int) (low >> 1 & 3u) <= scale;
+                tab[k * kOccCtaThreads] = (int) ((e >> 5) & 0xfffffffu) << 1 | (scale < (int) (low >> 3 & 3u) ? 1 : 0);
+            }
+            if (known)
+                have = fine;
+        }
+        const bool seek = have && !known;
+        if (__any_sync(kOccWarp, seek)) {
 #pragma unroll 1
-        for (int k = 0; k < 8; ++k) {
-            const bool look = have && (k & ~two) == 0;
-            if (!__any_sync(kOccWarp, look))
-                continue;
-            const int slot = occ_seek_warp(m, c, b0 + ((k & 1) ? stride : 0), b1 + ((k & 2) ? stride : 0),
-                                           b2 + ((k & 4) ? stride : 0), look);
-            if (look) {
-                have = slot != -1 && !(slot_is_block(slot) && c.cur > scale);
-                tab[k * kOccCtaThreads] = slot_is_block(slot) ? (slot_block(slot) << 1) | (scale < c.fin ? 1 : 0)
-                                                              : (occ_valid(c.nd) ? -1 : -2);
+            for (int k = 0; k < 8; ++k) {
+                const bool look = seek && have && (k & ~two) == 0;
+                if (!__any_sync(kOccWarp, look))
+                    continue;
+                const int slot = occ_seek_warp(m, c, b0 + ((k & 1) ? stride : 0), b1 + ((k & 2) ? stride : 0),
+                                               b2 + ((k & 4) ? stride : 0), look);
+                if (look) {
+                    have = slot != -1 && !(slot_is_block(slot) && c.cur > scale);
+                    tab[k * kOccCtaThreads] = slot_is_block(slot) ? (slot_block(slot) << 1) | (scale < c.fin ? 1 : 0)
+                                                                  : (occ_valid(c.nd) ? -1 : -2);
+                }
             }
         }
         bool valid = true;
