@@ -1542,8 +1542,8 @@ __device__ void occ_propagate_block(const OccDevice& m, int b, int lane)
 // freeBlock on the freed blocks and updateBlock on the carver's blocks (disjoint: the carver does not
 // descend below a free-space node), then the block's own propagation, one warp per block, all maps. A
 // block's propagation needs that block alone: in a stage of its own it read everything again (320x240: 42 +
-// 33 us as two launches, 57 as one; eight 1024x64 LiDAR maps: 102 + 64 and 127). The carver's blocks also put their parents in the first propagation
-// set (propagateToRoot's seeds).
+// 33 us as two launches, 57 as one; eight 1024x64 LiDAR maps: 102 + 64 and 127). The carver's blocks also
+// put their parents in the first propagation set (propagateToRoot's seeds).
 __device__ void occ_blocks_stage(const OccLaunch& L, int bid, int nbid)
 {
     __shared__ int pre[kOccMaxBatch + 1];

@@ -268,7 +268,7 @@ constexpr uint64_t kOccNearEmpty = ~0ull; // no entry: a slot is less
 
 // The leaf at a voxel (masked to the map) for the lanes with `need` set, from level L of the path down: its
 // slot, and level | current scale << 4 | finest << 8 | (the path's new lowest level, 0: not walked) << 12. A
-// function of its own, for the code's size: the rays that it serves are few and wait for instructions.
+// function of its own, for the code's size: its callers are many and its rays few.
 static __device__ __noinline__ int2 occ_find_warp(const OccDevice& m, uint64_t* near, int* path, int xm, int ym, int zm, int L,
                                                   bool need)
 {
@@ -868,7 +868,8 @@ __device__ __forceinline__ bool occ_raycast(const OccDevice& m, OccCursor& c, co
         const unsigned events = occ_sample_votes<kLanes>(take && there && (find ? has : !has || fk > -0.2f));
         const unsigned gone = occ_sample_votes<kLanes>(!there), data_bits = occ_sample_votes<kLanes>(has);
         const int e = events ? __ffs(events) - 1 : kLanes - 1; // the sample to act on, or the last one
-        const float t_e = occ_sample_from<kLanes>(tk, e), f_e = occ_sample_from<kLanes>(fk, e), t_b = occ_sample_from<kLanes>(tk, e - 1), f_b = occ_sample_from<kLanes>(fk, e - 1);
+        const float t_e = occ_sample_from<kLanes>(tk, e), f_e = occ_sample_from<kLanes>(fk, e);
+        const float t_b = occ_sample_from<kLanes>(tk, e - 1), f_b = occ_sample_from<kLanes>(fk, e - 1);
         pass = __shfl_sync(kOccWarp, pass, threadIdx.x | (kLanes - 1));
         if (take) {
             if (events) {
@@ -1006,14 +1007,16 @@ __device__ __forceinline__ bool occ_raycast(const OccDevice& m, OccCursor& c, co
 //
 // Why: rays along the edge of what has been seen take 50 to 120 turns of the loop, the others 7, and lie
 // together. Four to a warp, 1 % of the warps were most of the time, with the rest of the GPU idle, and all
-// of them waited for instructions (65 KB of code as one kernel; 42, 50 and 19 as three). A view of a room,
+// of them waited for instructions (2 stall cycles an issue with 65 KB of code in one kernel, 0.3 to 0.6
+// now). A view of a room,
 // 2 cm, with its integration: 320x240 820 us as one kernel, 744 with the rays put aside, 704 with the normals
-// apart too; a 160x120 view after eight LiDAR scans 577, 590 and 567.
+// apart too; a 160x120 view after eight LiDAR scans 577, 590 and 567. (8 CTAs an SM for the rays: 640x480 1411
+// to 1392 us, with the 72 registers they would take 7.)
 constexpr float kOccSuspendedMark = 2.0f, kOccHitMark = 3.0f;
 template <bool RESUME>
-__global__ void __launch_bounds__(kOccCtaThreads) occ_raycast_kernel(const __grid_constant__ OccDevice m, OccRes r, Pinhole s,
-                                                                     Tf T_WS, float* __restrict__ pts,
-                                                                     float* __restrict__ nrm, int8_t* __restrict__ scale)
+__global__ void __launch_bounds__(kOccCtaThreads, RESUME ? 5 : 8)
+    occ_raycast_kernel(const __grid_constant__ OccDevice m, OccRes r, Pinhole s, Tf T_WS, float* __restrict__ pts,
+                       float* __restrict__ nrm, int8_t* __restrict__ scale)
 {
     grid_dep_wait();
     __shared__ int sh_path[kOccPathLevels * kOccCtaThreads];
