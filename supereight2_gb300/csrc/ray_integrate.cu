@@ -39,6 +39,7 @@
 
 #include "occupancy.cuh"
 #include "pipeline.cuh"
+#include "ray_voxel.cuh"
 #include "se_gpu_internal.cuh"
 
 namespace se_gpu {
@@ -891,25 +892,6 @@ __device__ __forceinline__ bool ri_sample(float range_diff, const RiRayF& R, con
     if (range_diff < -R.three_sigma)
         sample = c.log_odd_min;
     return range_diff < -R.three_sigma || range_diff < R.tau / 2.0f || range_diff < R.tau;
-}
-
-// inv: 1 / w for the integer weights w < kRiInv, correctly rounded: the quotient by w from it and one
-// residual is the correctly rounded one (Markstein's theorem, as div_res in se_gpu_internal.cuh).
-constexpr int kRiInv = 32;
-
-__device__ __forceinline__ void ri_update_voxel(OccD& d, float sample, const OccFieldConfig& c, const float* inv)
-{
-    if (d.weight < c.max_weight)
-        d.weight = d.weight + 1.0f;
-    const float w = d.weight, x = d.occ * (w - 1.0f) + sample;
-    if (w < (float) kRiInv && fabsf(x) >= 0x1p-100f && fabsf(x) < 0x1p100f) {
-        const float i = inv[(int) w], q = x * i;
-        d.occ = fmaf(fmaf(-q, w, x), i, q);
-    }
-    else {
-        d.occ = x / w;
-    }
-    d.observed = 1;
 }
 
 // updateBlock (ray_integrator_impl.hpp:232-300)
