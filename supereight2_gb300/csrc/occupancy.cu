@@ -7,6 +7,7 @@
 #include <cstring>
 #include <vector>
 
+#include "occ_march.cuh"
 #include "occupancy.cuh"
 #include "pipeline.cuh"
 #include "profile.cuh"
@@ -169,52 +170,6 @@ __device__ __forceinline__ OccD occ_get_data_voxel(const OccDevice& m, OccCursor
     if (slot_is_block(slot))
         return blk_mean(m, slot_block(slot), c.cur)[blk_voxel_idx(x, y, z, c.cur)];
     return c.nd;
-}
-
-// x / res, correctly rounded, from the reciprocal and one residual (div_res in se_gpu_internal.cuh)
-struct OccRes {
-    float res, inv;
-    int translation; // T_MW is a translation
-};
-__device__ __forceinline__ float occ_div_res(const OccRes& r, float x)
-{
-    if (!(fabsf(x) >= 0x1p-100f && fabsf(x) < 0x1p100f))
-        return x / r.res;
-    const float q = x * r.inv;
-    return fmaf(fmaf(-q, r.res, x), r.inv, q);
-}
-
-__device__ __forceinline__ bool occ_in_map(const OccDevice& m, F3 p)
-{
-    return p.x >= 0.0f && p.x < m.dim && p.y >= 0.0f && p.y < m.dim && p.z >= 0.0f && p.z < m.dim;
-}
-
-// The same for a sample of the march: a coordinate below 2^-100 or beyond 2^100 may come out an ulp off,
-// which neither its voxel nor its place in a cell (less half a voxel) can tell.
-__device__ __forceinline__ F3 occ_sample_voxel(const OccRes& r, F3 p)
-{
-    const F3 q = f3(p.x * r.inv, p.y * r.inv, p.z * r.inv);
-    return f3(fmaf(fmaf(-q.x, r.res, p.x), r.inv, q.x), fmaf(fmaf(-q.y, r.res, p.y), r.inv, q.y),
-              fmaf(fmaf(-q.z, r.res, p.z), r.inv, q.z));
-}
-
-// T_MW p; translation: T_MW's rotation is exactly the identity (the products by 1 and 0 change nothing
-// but the sign of a zero).
-__device__ __forceinline__ F3 occ_to_map(const OccDevice& m, const OccRes& r, F3 p)
-{
-    if (r.translation)
-        return f3(p.x + m.T_MW.t[0], p.y + m.T_MW.t[1], p.z + m.T_MW.t[2]);
-    return apply(m.T_MW, p);
-}
-
-__device__ __forceinline__ F3 occ_voxel_f(const OccRes& r, F3 p_M)
-{
-    return f3(occ_div_res(r, p_M.x), occ_div_res(r, p_M.y), occ_div_res(r, p_M.z));
-}
-
-__device__ __forceinline__ F3 occ_to_voxel_f(const OccDevice& m, const OccRes& r, F3 p_W)
-{
-    return occ_voxel_f(r, apply(m.T_MW, p_W));
 }
 
 constexpr unsigned kOccWarp = 0xffffffffu;
@@ -532,23 +487,6 @@ __device__ __forceinline__ bool occ_grad(const OccDevice& m, OccCursor& c, F3 vf
     return ok;
 }
 
-// The samples t + step, t + 2 step, ... (at most kOccSkipMax of them) that are certain to lie in the
-// cursor's box, from the voxel position v of sample t and the ray's direction dv in voxels per unit
-// of t: the distance to the box's faces less a quarter voxel, which bounds the float error of a
-// sample position and of kOccSkipMax accumulated steps in a map of 8192 voxels a side, and less one
-// whole step.
-constexpr int kOccSkipMax = 256;
-__device__ __forceinline__ int occ_box_steps(const OccCursor& c, F3 v, F3 dv, float step)
-{
-    const float size = (float) (~c.mask + 1);
-    const float rx = dv.x > 0.0f ? (float) c.bx + size - v.x : v.x - (float) c.bx;
-    const float ry = dv.y > 0.0f ? (float) c.by + size - v.y : v.y - (float) c.by;
-    const float rz = dv.z > 0.0f ? (float) c.bz + size - v.z : v.z - (float) c.bz;
-    const float lim = fminf(fminf((rx - 0.25f) / fabsf(dv.x), (ry - 0.25f) / fabsf(dv.y)), (rz - 0.25f) / fabsf(dv.z));
-    const float n = fminf(lim / step, (float) kOccSkipMax) - 1.0f;
-    return n > 0.0f ? (int) n : 0; // also 0 for a NaN
-}
-
 // Whether occ_interp has a value at vf, each lane with `run` set for its own point. The blocks of a cell's
 // corners (one, or two along an axis the cell crosses a block's face on) are looked up into `tab` (the
 // lane's 8 words of shared memory, kOccCtaThreads apart): a block and whether its initial data holds at the
@@ -855,7 +793,7 @@ __device__ __forceinline__ bool occ_raycast(const OccDevice& m, OccCursor& c, co
             has = occ_valid(data);
             fk = occ_field(data);
             if (find && !has && lane == kLanes - 1 && !slot_is_block(c.slot))
-                pass = occ_box_steps(c, vk, dv, step);
+                pass = occ_box_steps(r, c.bx, c.by, c.bz, ~c.mask + 1, vk, dv, step);
         }
         if constexpr (RESUME) {
             const bool probe = find && has && failed >= kOccTries;
@@ -1116,15 +1054,13 @@ se_gpu_status occ_raycast_volume(const se_gpu_occ_map* om, const se_gpu_pinhole&
 {
     const Pinhole s = make_pinhole(sensor);
     dim3 grid((s.w + 3) / 4, (s.h + 3) / 4);
-    OccRes r = {om->dev.res, 1.0f / om->dev.res, 1};
-    for (int i = 0; i < 9; ++i)
-        if (om->dev.T_MW.R[i] != ((i % 4 == 0) ? 1.0f : 0.0f))
-            r.translation = 0;
+    const Tf T_WS = tf_from16(T_WS16);
+    const OccRes r = occ_res(om->dev, f3(T_WS.t[0], T_WS.t[1], T_WS.t[2]));
     ProfScope ps(kProfRaycast, stream);
-    launch_chained(occ_raycast_kernel<false>, grid, kOccCtaThreads, stream, om->dev, r, s, tf_from16(T_WS16), pts, nrm, scale);
+    launch_chained(occ_raycast_kernel<false>, grid, kOccCtaThreads, stream, om->dev, r, s, T_WS, pts, nrm, scale);
     constexpr int kWarps = kOccCtaThreads / 32;
     launch_chained(occ_raycast_kernel<true>, (s.w * s.h + kWarps - 1) / kWarps, kOccCtaThreads, stream, om->dev, r, s,
-                   tf_from16(T_WS16), pts, nrm, scale);
+                   T_WS, pts, nrm, scale);
     launch_chained(occ_normal_kernel, grid, kOccCtaThreads, stream, om->dev, r, s.w, s.h, pts, nrm);
     SE_CUDA_TRY(cudaGetLastError());
     return SE_GPU_OK;
