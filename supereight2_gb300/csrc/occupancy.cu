@@ -1,6 +1,7 @@
 // occupancy.cu — multi-resolution occupancy maps (Map<Data<Occupancy>, Res::Multi, 8>): the
 // map's pools (creation, destruction, checks, downloads) and the raycast over the octree
 // (raycaster_impl.hpp:32-452). Integration lives in occ_integrate.cu.
+#include <algorithm>
 #include <cfloat>
 #include <climits>
 #include <cmath>
@@ -951,6 +952,20 @@ __device__ __forceinline__ bool occ_raycast(const OccDevice& m, OccCursor& c, co
 // apart too; a 160x120 view after eight LiDAR scans 577, 590 and 567. (8 CTAs an SM for the rays: 640x480 1411
 // to 1392 us, with the 72 registers they would take 7.)
 constexpr float kOccSuspendedMark = 2.0f, kOccHitMark = 3.0f;
+
+// The pixel of a CTA's warp and group in a grid of occ_tiles: 4 x 4 pixels a CTA, the rows of CTAs along y and,
+// past the 65,535 of a grid's y (262,140 pixels), along z.
+__device__ __forceinline__ void occ_pixel_of(int warp, int ray, int& x, int& y)
+{
+    x = blockIdx.x * 4 + (warp & 1) * 2 + (ray & 1);
+    y = (blockIdx.z * gridDim.y + blockIdx.y) * 4 + (warp >> 1) * 2 + (ray >> 1);
+}
+static dim3 occ_tiles(int w, int h)
+{
+    const unsigned rows = ((unsigned) h + 3) / 4, y = std::min(rows, 65535u);
+    return dim3(((unsigned) w + 3) / 4, y, (rows + y - 1) / y);
+}
+
 template <bool RESUME>
 __global__ void __launch_bounds__(kOccCtaThreads, RESUME ? 5 : 8)
     occ_raycast_kernel(const __grid_constant__ OccDevice m, OccRes r, Pinhole s, Tf T_WS, float* __restrict__ pts,
@@ -967,15 +982,14 @@ __global__ void __launch_bounds__(kOccCtaThreads, RESUME ? 5 : 8)
     const int warp = threadIdx.x >> 5, ray = (threadIdx.x >> 3) & 3, lane = threadIdx.x & 7;
     int x, y;
     if constexpr (RESUME) {
-        const int i = blockIdx.x * (kOccCtaThreads / 32) + warp;
-        if (i >= s.w * s.h || nrm[3 * (size_t) i] != kOccSuspendedMark)
+        const size_t i = (size_t) blockIdx.x * (kOccCtaThreads / 32) + warp;
+        if (i >= (size_t) s.w * s.h || nrm[3 * i] != kOccSuspendedMark)
             return;
-        x = i % s.w;
-        y = i / s.w;
+        x = (int) (i % s.w);
+        y = (int) (i / s.w);
     }
     else {
-        x = blockIdx.x * 4 + (warp & 1) * 2 + (ray & 1);
-        y = blockIdx.y * 4 + (warp >> 1) * 2 + (ray >> 1);
+        occ_pixel_of(warp, ray, x, y);
     }
     const bool in_image = x < s.w && y < s.h; // rays past the edge stay for the warp's votes
     OccCursor c;
@@ -1029,8 +1043,8 @@ __global__ void __launch_bounds__(kOccCtaThreads) occ_normal_kernel(const __grid
     __shared__ int sh_path[kOccPathLevels * kOccCtaThreads];
     __shared__ float sh_grad[kOccCtaThreads / 8][33];
     const int warp = threadIdx.x >> 5, ray = (threadIdx.x >> 3) & 3, lane = threadIdx.x & 7;
-    const int x = blockIdx.x * 4 + (warp & 1) * 2 + (ray & 1);
-    const int y = blockIdx.y * 4 + (warp >> 1) * 2 + (ray >> 1);
+    int x, y;
+    occ_pixel_of(warp, ray, x, y);
     const size_t idx = (size_t) x + (size_t) y * w;
     const bool is_hit = x < w && y < h && nrm[3 * idx] == kOccHitMark;
     if (!__any_sync(kOccWarp, is_hit))
@@ -1053,13 +1067,14 @@ se_gpu_status occ_raycast_volume(const se_gpu_occ_map* om, const se_gpu_pinhole&
                                  float* pts, float* nrm, int8_t* scale, cudaStream_t stream)
 {
     const Pinhole s = make_pinhole(sensor);
-    dim3 grid((s.w + 3) / 4, (s.h + 3) / 4);
+    const dim3 grid = occ_tiles(s.w, s.h);
     const Tf T_WS = tf_from16(T_WS16);
     const OccRes r = occ_res(om->dev, f3(T_WS.t[0], T_WS.t[1], T_WS.t[2]));
     ProfScope ps(kProfRaycast, stream);
     launch_chained(occ_raycast_kernel<false>, grid, kOccCtaThreads, stream, om->dev, r, s, T_WS, pts, nrm, scale);
     constexpr int kWarps = kOccCtaThreads / 32;
-    launch_chained(occ_raycast_kernel<true>, (s.w * s.h + kWarps - 1) / kWarps, kOccCtaThreads, stream, om->dev, r, s,
+    const unsigned warps_ctas = (unsigned) (((size_t) s.w * s.h + kWarps - 1) / kWarps);
+    launch_chained(occ_raycast_kernel<true>, warps_ctas, kOccCtaThreads, stream, om->dev, r, s,
                    T_WS, pts, nrm, scale);
     launch_chained(occ_normal_kernel, grid, kOccCtaThreads, stream, om->dev, r, s.w, s.h, pts, nrm);
     SE_CUDA_TRY(cudaGetLastError());
