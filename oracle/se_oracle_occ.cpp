@@ -1643,21 +1643,31 @@ static inline bool occ_interp_W(const so_occ_map& m, V3 p_W, float& out, int* sc
     return occ_interp(m, apply(m.T_MW, p_W) / m.res, 0, out, scale);
 }
 
+/* The longest run of points with data but no interpolation that a search of this thread has met. */
+static thread_local int longest_misses;
+
 /* find_valid_point (raycaster_impl.hpp:32-70) */
 static bool find_valid_point(const so_occ_map& m, V3 o, V3 d, float step, float t_max, float& t, V3& point_W,
                              float& value)
 {
     bool has = false;
+    int misses = 0;
+    const auto interp = [&](V3 q) {
+        const bool ok = occ_interp_W(m, q, value, nullptr);
+        misses = ok ? 0 : misses + 1;
+        longest_misses = std::max(longest_misses, misses);
+        return ok;
+    };
     V3 p = o + t * d;
     if (occ_contains(m, p) && occ_valid(occ_get_data(m, p)))
-        has = occ_interp_W(m, p, value, nullptr);
+        has = interp(p);
     while (!has) {
         t += step;
         if (t > t_max)
             return false;
         p = o + t * d;
         if (occ_contains(m, p) && occ_valid(occ_get_data(m, p)))
-            has = occ_interp_W(m, p, value, nullptr);
+            has = interp(p);
     }
     point_W = p;
     return true;
@@ -2737,6 +2747,24 @@ long long so_occ_nodes(const so_occ_map* mp, int32_t* coords, float* min_data, f
 }
 
 int so_occ_map_size(const so_occ_map* m) { return m->octree.size; }
+
+void so_occ_raycast_misses(const so_occ_map* mp, const so_pinhole* sensor_c, const float T_WS_m[16], int* misses)
+{
+    const so_occ_map& m = *mp;
+    const Pinhole s = make_pinhole(sensor_c);
+    const Tf T_WS = tf_from16(T_WS_m);
+#pragma omp parallel for schedule(dynamic, 4)
+    for (int y = 0; y < s.h; y++) {
+        for (int x = 0; x < s.w; x++) {
+            const V3 ray_S = back_project(s, (float) x, (float) y);
+            V3 hit;
+            int scale;
+            longest_misses = 0;
+            raycast_occ(m, v3(T_WS.t[0], T_WS.t[1], T_WS.t[2]), rot(T_WS, normalized(ray_S)), far_dist(s, ray_S), hit, scale);
+            misses[(size_t) x + (size_t) y * (size_t) s.w] = longest_misses;
+        }
+    }
+}
 
 /* raycaster::raycast_volume for occupancy maps (raycaster_impl.hpp:537-627): normals are the
  * negated normalised field gradient (normals_along_gradient is false for occupancy). */
