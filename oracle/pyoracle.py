@@ -80,7 +80,7 @@ def lib():
             "so_occ_blocks": (None, [vp, vp, vp, vp, vp, vp, vp]),
             "so_occ_nodes": (C.c_longlong, [vp, vp, vp, vp, vp]),
             "so_occ_aabb": (C.c_int, [vp, i32p, i32p]),
-            "so_occ_raycast_misses": (None, [vp, C.POINTER(Pinhole), f32p, i32p]),
+            "so_occ_raycast_misses": (None, [vp, C.POINTER(Pinhole), f32p, f32p, f32p, i8p, i32p]),
             "so_occ_raycast_volume": (None, [vp, C.POINTER(Pinhole), f32p, f32p, f32p, i8p]),
             "so_occ_depth_sigma": (None, [f32p, C.c_int, C.c_float, f32p]),
             "so_occ_pooling_image": (C.c_int, [f32p, C.c_int, C.c_int, vp, C.POINTER(C.c_float)]),
@@ -202,20 +202,19 @@ class OracleOccMap:
             self.h = lib().so_occ_map_create(d, float(res), tmw)
         self.res = float(res)
 
-    def raycast(self, sensor, T_WS):
+    def raycast(self, sensor, T_WS, misses=None):
+        """misses: an int32 array of the image's size, set to the longest run of points with data but no
+        interpolation in a search of each pixel's ray."""
         n = sensor.width * sensor.height
         pts = np.zeros((sensor.height, sensor.width, 3), np.float32)
         nrm = np.zeros((sensor.height, sensor.width, 3), np.float32)
         scale = np.zeros((sensor.height, sensor.width), np.int8)
-        lib().so_occ_raycast_volume(self.h, C.byref(sensor), _m16(T_WS), pts.reshape(n * 3),
-                                    nrm.reshape(n * 3), scale.reshape(n))
+        out = (self.h, C.byref(sensor), _m16(T_WS), pts.reshape(n * 3), nrm.reshape(n * 3), scale.reshape(n))
+        if misses is None:
+            lib().so_occ_raycast_volume(*out)
+        else:
+            lib().so_occ_raycast_misses(*out, misses.reshape(n))
         return pts, nrm, scale
-
-    def raycast_misses(self, sensor, T_WS):
-        """Per pixel, the longest run of points with data but no interpolation in a search of its ray."""
-        misses = np.zeros((sensor.height, sensor.width), np.int32)
-        lib().so_occ_raycast_misses(self.h, C.byref(sensor), _m16(T_WS), misses.reshape(-1))
-        return misses
 
     def get_data(self, p):
         out = np.zeros(3, np.float32)

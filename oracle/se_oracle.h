@@ -193,9 +193,10 @@ int so_occ_aabb(const so_occ_map* map, int32_t mn[3], int32_t mx[3]);
 /* raycaster::raycast_volume for an occupancy map (raycaster_impl.hpp:32-452,537-627). */
 void so_occ_raycast_volume(const so_occ_map* map, const so_pinhole* sensor, const float T_WS[16],
                            float* pts_W, float* nrm_W, int8_t* scale);
-/* For each pixel of such a raycast, the longest run of points in one of its ray's searches that have
- * data but no interpolation. */
-void so_occ_raycast_misses(const so_occ_map* map, const so_pinhole* sensor, const float T_WS[16], int* misses);
+/* The same with, for each pixel, the longest run of points in one of its ray's searches that have data
+ * but no interpolation. */
+void so_occ_raycast_misses(const so_occ_map* map, const so_pinhole* sensor, const float T_WS[16],
+                           float* pts_W, float* nrm_W, int8_t* scale, int* misses);
 /* A spinning LiDAR (the reference's OusterLidar): equiangular columns over 360 degrees of azimuth
  * (clockwise from +x), rows linear in elevation from elevation_max_deg (row 0) down to
  * elevation_min_deg; the range image holds ranges in metres (<= 0: no return). */

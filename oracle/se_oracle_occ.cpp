@@ -2748,28 +2748,10 @@ long long so_occ_nodes(const so_occ_map* mp, int32_t* coords, float* min_data, f
 
 int so_occ_map_size(const so_occ_map* m) { return m->octree.size; }
 
-void so_occ_raycast_misses(const so_occ_map* mp, const so_pinhole* sensor_c, const float T_WS_m[16], int* misses)
-{
-    const so_occ_map& m = *mp;
-    const Pinhole s = make_pinhole(sensor_c);
-    const Tf T_WS = tf_from16(T_WS_m);
-#pragma omp parallel for schedule(dynamic, 4)
-    for (int y = 0; y < s.h; y++) {
-        for (int x = 0; x < s.w; x++) {
-            const V3 ray_S = back_project(s, (float) x, (float) y);
-            V3 hit;
-            int scale;
-            longest_misses = 0;
-            raycast_occ(m, v3(T_WS.t[0], T_WS.t[1], T_WS.t[2]), rot(T_WS, normalized(ray_S)), far_dist(s, ray_S), hit, scale);
-            misses[(size_t) x + (size_t) y * (size_t) s.w] = longest_misses;
-        }
-    }
-}
-
 /* raycaster::raycast_volume for occupancy maps (raycaster_impl.hpp:537-627): normals are the
  * negated normalised field gradient (normals_along_gradient is false for occupancy). */
-void so_occ_raycast_volume(const so_occ_map* mp, const so_pinhole* sensor_c, const float T_WS_m[16], float* pts_W,
-                           float* nrm_W, int8_t* scale)
+static void raycast_image(const so_occ_map* mp, const so_pinhole* sensor_c, const float T_WS_m[16], float* pts_W,
+                          float* nrm_W, int8_t* scale, int* misses)
 {
     const so_occ_map& m = *mp;
     const Pinhole s = make_pinhole(sensor_c);
@@ -2783,6 +2765,7 @@ void so_occ_raycast_volume(const so_occ_map* mp, const so_pinhole* sensor_c, con
             const V3 dir_W = rot(T_WS, normalized(ray_S));
             V3 hit;
             int sc = 0;
+            longest_misses = 0;
             V3 p = v3(0.0f, 0.0f, 0.0f), n = v3(0.0f, 0.0f, 0.0f);
             if (raycast_occ(m, origin, dir_W, far_dist(s, ray_S), hit, sc)) {
                 p = hit;
@@ -2799,6 +2782,8 @@ void so_occ_raycast_volume(const so_occ_map* mp, const so_pinhole* sensor_c, con
             else {
                 sc = 0;
             }
+            if (misses)
+                misses[idx] = longest_misses;
             scale[idx] = (int8_t) sc;
             pts_W[3 * idx + 0] = p.x;
             pts_W[3 * idx + 1] = p.y;
@@ -2808,6 +2793,18 @@ void so_occ_raycast_volume(const so_occ_map* mp, const so_pinhole* sensor_c, con
             nrm_W[3 * idx + 2] = n.z;
         }
     }
+}
+
+void so_occ_raycast_volume(const so_occ_map* m, const so_pinhole* sensor, const float T_WS[16], float* pts_W,
+                           float* nrm_W, int8_t* scale)
+{
+    raycast_image(m, sensor, T_WS, pts_W, nrm_W, scale, nullptr);
+}
+
+void so_occ_raycast_misses(const so_occ_map* m, const so_pinhole* sensor, const float T_WS[16], float* pts_W,
+                           float* nrm_W, int8_t* scale, int* misses)
+{
+    raycast_image(m, sensor, T_WS, pts_W, nrm_W, scale, misses);
 }
 
 int so_occ_aabb(const so_occ_map* m, int32_t mn[3], int32_t mx[3])

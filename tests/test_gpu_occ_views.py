@@ -61,8 +61,8 @@ def test_views_with_hits(oracle, gpu, width, height, dim, res, angle, back, orig
         integ.integrateDepth(k, torch.from_numpy(depth).cuda(), gpu.PinholeCamera(**SPEC), T)
     gm.check()
     view, V = _view(width, height, dim, origin, angle, back)
-    op, on, osc = om.raycast(oracle.pinhole(**view), V)
-    misses = om.raycast_misses(oracle.pinhole(**view), V)
+    misses = np.zeros((height, width), np.int32)
+    op, on, osc = om.raycast(oracle.pinhole(**view), V, misses)
     pts = torch.full((height, width, 3), 7.0, device="cuda")
     nrm = torch.full_like(pts, 7.0)
     sc = torch.full((height, width), 7, dtype=torch.int8, device="cuda")
