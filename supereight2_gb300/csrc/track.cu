@@ -439,6 +439,13 @@ __device__ __forceinline__ void bar_named(int id, int nthreads)
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
+// x 2^e by the exponent field (no FP64 instruction): 0 below the normal range, no finite number above it.
+__device__ __forceinline__ double mul_pow2(double x, int e)
+{
+    const int hi = __double2hiint(x), f = (hi >> 20) & 0x7ff, fe = min(f + e, 0x7ff);
+    return f == 0 || fe <= 0 ? 0.0 : __hiloint2double((hi & 0x800fffff) | (fe << 20), __double2loint(x));
+}
+
 // Solves C x = b (C symmetric, the packed upper triangle of the newReduce layout in sh_val[7..27],
 // b = sh_val[1..6], icp.cpp:15-41), forms exp(x) (math_util_impl.hpp:117-174 in Rodrigues form:
 // R = I + A W + B W^2, V = I + B W + C W^2, W = hat(omega), translation V rho) and composes
@@ -459,7 +466,14 @@ __device__ __noinline__ void icp_tail(const double* sh_val, const double* sh_pos
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (warp < 2) {
         // elimination: entry e = 21 warp + lane (lanes < 21) is (r, c) of the 6 x 7 system; each
-        // lane keeps its entry in a register and publishes it for the other rows each step
+        // lane keeps its entry in a register and publishes it for the other rows each step. The rows
+        // are multiplied by each pivot in place of being divided by it. The pivot is brought into
+        // [1, 2) for that, by a power of two that goes into the whole row: no digit of a result
+        // changes, and the entries keep their size. (Without it their exponents doubled from step to
+        // step; from 220,000 inliers on they left FP64's range, and the frame was lost. The integer
+        // operations fill a wait for the other operands: track() 173.9 us without them, 173.6 with.
+        // For the third and the fifth pivot only, as few as will do, it took 188.3 against 184.6: the
+        // branch costs more.)
         const bool gj = lane < 21;
         const int e = warp * 21 + lane, r = e / 7, c = e % 7;
         double a = 0.0;
@@ -476,11 +490,13 @@ __device__ __noinline__ void icp_tail(const double* sh_val, const double* sh_pos
             const double* Mi = M[j & 1];
             double* Mo = M[(j + 1) & 1];
             if (gj) {
-                const double d = Mi[7 * j + j];
+                const double pivot = Mi[7 * j + j];
+                const int ed = ((__double2hiint(pivot) >> 20) & 0x7ff) - 1023;
+                const double d = mul_pow2(pivot, -ed), x = mul_pow2(Mi[7 * r + j], -ed);
                 if (r != j)
-                    a = c == j ? 0.0 : fma(d, a, -(Mi[7 * r + j] * Mi[7 * j + c]));
+                    a = c == j ? 0.0 : fma(d, a, -(x * Mi[7 * j + c]));
                 Mo[e] = a;
-                if (e == 0 && !pivot_ok(d))
+                if (e == 0 && !pivot_ok(pivot))
                     sh_ok = 0;
             }
             bar_named(1, 64);
