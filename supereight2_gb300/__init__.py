@@ -209,8 +209,9 @@ def _stream(stream):
         return C.c_void_p(int(stream))
     import torch
     # The handle without a Stream object where this torch has it (two short calls: 12 us, 20 without).
-    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-    if raw is None:
+    try:
+        raw = torch._C._cuda_getCurrentRawStream
+    except AttributeError:
         return C.c_void_p(torch.cuda.current_stream().cuda_stream)
     return C.c_void_p(raw(torch.cuda.current_device()))
 

@@ -81,22 +81,6 @@ __device__ __forceinline__ int mr_block_of(const MapDevice& m, int vx, int vy, i
                                 | (size_t) (vx >> 3)]);
 }
 
-// visitor::getData multi-res (visitor_impl.hpp:704-717): the data at the block's current scale,
-// or the default data (tsdf 1, weight 0) where no block is allocated. A block that has never
-// been integrated holds the default data.
-template <int S>
-__device__ __forceinline__ void mr_get_data(const MapDevice& m, int vx, int vy, int vz, float& t, float& w)
-{
-    const int b = mr_block_of(m, vx, vy, vz);
-    int cur = b < 0 ? -1 : (int) m.block_scale[2 * b];
-    if (cur < 0) {
-        t = 1.0f;
-        w = 0.0f;
-        return;
-    }
-    mr_load_data<S>(m, b, mr_index(vx & 7, vy & 7, vz & 7, cur), t, w);
-}
-
 // The block last looked up by a thread, with its current scale (-1 before its first update or where
 // nothing is allocated).
 struct MrCache {
@@ -116,7 +100,9 @@ __device__ __forceinline__ void mr_lookup(const MapDevice& m, MrCache& c, int vx
     }
 }
 
-// mr_get_data through the cache.
+// visitor::getData multi-res (visitor_impl.hpp:704-717): the data at the block's current scale, or the default
+// data (tsdf 1, weight 0) where no block is allocated. A block that has never been integrated holds the default
+// data.
 template <int S>
 __device__ __forceinline__ void mr_get_data(const MapDevice& m, MrCache& c, int vx, int vy, int vz, float& t, float& w)
 {

@@ -31,7 +31,7 @@ constexpr int kOccPathLevels = 10;  // levels 4..13: nodes of 16^3 to 8192^3 vox
 
 // A lane's place in the octree. Successive lookups lie in the same leaf octant or next to it, so each
 // starts from what the last one found instead of from the root:
-//   - the box of the last leaf lookup (occ_leaf's answer is the same for every voxel in it), with
+//   - the box of the last leaf lookup (the answer is the same for every voxel in it), with
 //     its block's scales or its node's data;
 //   - the nodes on the path to the last voxel descended to, one per level, in shared memory
 //     (path[L * kOccCtaThreads], this thread's column): a lookup restarts at the deepest node that
@@ -42,7 +42,7 @@ struct OccCursor {
     uint64_t* near; // a whole warp's leaves, see occ_seek_warp
     int px, py, pz; // the voxel of the path (masked to the map)
     int low;        // path entries of levels low..log2_size are valid
-    int slot;       // occ_leaf's answer inside the box (bx, by, bz) / mask
+    int slot;       // fetcher::leaf's answer inside the box (bx, by, bz) / mask: a slot, or -1
     int bx, by, bz, mask;
     int cur, fin;   // a block's current and finest allocated scale
     OccD nd;        // a leaf node's data (default for -1)

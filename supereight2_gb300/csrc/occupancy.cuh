@@ -258,23 +258,6 @@ __device__ __forceinline__ OccD node_data(const OccDevice& m, int n)
     return (mx.observed && node_is_leaf(m, n)) ? mx : occ_default();
 }
 
-// fetcher::leaf: slot of the block holding the voxel, the deepest node on its path if that node
-// has no children, or -1.
-__device__ __forceinline__ int occ_leaf(const OccDevice& m, int x, int y, int z)
-{
-    int n = 0;
-    for (int cs = m.size >> 1; cs >= 8; cs >>= 1) {
-        const int idx = ((x & cs) > 0) + 2 * ((y & cs) > 0) + 4 * ((z & cs) > 0);
-        const int ch = m.node_child[8 * (size_t) n + idx];
-        if (ch == -1)
-            return node_is_leaf(m, n) ? n : -1;
-        if (slot_is_block(ch))
-            return ch;
-        n = ch;
-    }
-    return n;
-}
-
 __device__ __forceinline__ int occ_voxel_idx(int ox, int oy, int oz, int s)
 {
     const int n = 8 >> s;

@@ -601,7 +601,9 @@ __device__ __forceinline__ void grid_dep_wait()
 // like the persistent ICP's), is never launched with this attribute. Early-scheduled CTAs hold
 // SM slots while they wait for their predecessor, and a grid barrier assumes that all of its
 // CTAs are resident at once. Such kernels get an ordinary (or cooperative) launch, which starts
-// only after the previous kernel has finished.
+// only after the previous kernel has finished. The one exception is a kernel whose CTAs wait only
+// for those of their own cluster (launch_clusters in occ_integrate.cu): a cluster is scheduled as a
+// whole, so its barrier always ends.
 template <typename... KArgs, typename... Args>
 inline void launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t stream, Args... args)
 {
