@@ -8,16 +8,17 @@
 //   pooling    DensePoolingImage<PinholeCamera | OusterLidar> levels 1.. of the depth and sigma
 //              images (dense_pooling_image_impl.hpp:56-213, 395-598), one launch per level
 //   root       DensePoolingImage::maxValue, VolumeCarver's max depth and the root's children
-//   carve      VolumeCarver (volume_carver_impl.hpp:46-537) breadth first, one launch per octree
-//              depth; a split node allocates its 8 children (Octree::allocateChildren) and queues
-//              them for the next depth
+//   carve      VolumeCarver (volume_carver_impl.hpp:46-537) breadth first, one launch for the root
+//              and the first depths, then one per octree depth; a split node allocates its 8 children
+//              (Octree::allocateChildren) and queues them for the next depth
 //   nodes      the carver's free-space nodes: AABB of the leaves, seeds of freeNodeRecurse
 //   free       Updater::freeNodeRecurse (multires_ofusion_updater_impl.hpp:550-600) one level of
 //              the free nodes' subtrees per launch
 //   blocks     Updater::freeBlock on the blocks below free nodes and Updater::updateBlock
-//              (:168-409) on the carver's blocks, one warp per block
-//   propagate  propagate_block_to_coarsest_scale on those blocks, then propagateToRoot (:129-164)
-//              one depth per launch from the blocks' parents up, with pruning, and the root
+//              (:168-409) on the carver's blocks, then propagate_block_to_coarsest_scale on each, one
+//              warp per block
+//   propagate  propagateToRoot (:129-164) from the blocks' parents up, with pruning: one depth per
+//              launch, the last depths and the root in one
 // The reference's recursion and OpenMP loops visit independent octants; the breadth-first
 // launches visit the same octants with the same per-octant computation, so the allocated
 // octree, the block lists (as sets) and every voxel agree with a serial run.
